@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "tof.cuh"
 
 namespace omb {
 
@@ -547,12 +548,23 @@ int omb_create(const omb_geometry_desc *desc, omb_handle **out) {
             (e = cudaMemcpy(h->d_ax, desc->ax_index, nb, cudaMemcpyHostToDevice)) != cudaSuccess)
             return fail(cuda_fail(e, "upload event indices"));
     }
-    if ((e = cudaMalloc(&h->d_tofc, kMaxTofBins * sizeof(float))) != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc tof"));
-    if ((e = cudaMemset(h->d_tofc, 0, kMaxTofBins * sizeof(float))) != cudaSuccess) return fail(cuda_fail(e, "clear tof"));
-    if (desc->tof_bins > 1 &&
-        (e = cudaMemcpy(h->d_tofc, desc->tof_centers, desc->tof_bins * sizeof(float), cudaMemcpyHostToDevice)) != cudaSuccess)
+    // the bin centres as given, in ascending order, and which bin each of those is
+    float tofc[3 * kMaxTofBins] = {};
+    int tofo[kMaxTofBins] = {};
+    if (desc->tof_bins > 1) {
+        std::copy(desc->tof_centers, desc->tof_centers + desc->tof_bins, tofc);
+        const float element = desc->fp_type == 4 && desc->bp_type == 4
+                                  ? desc->dL
+                                  : std::max(desc->dL, std::sqrt(g.dx * g.dx + g.dy * g.dy + g.dz * g.dz));
+        tof_setup(t, tofc, tofc + kMaxTofBins, tofo, element);
+        std::memcpy(tofc + 2 * kMaxTofBins, tofo, sizeof tofo);
+    }
+    if ((e = cudaMalloc(&h->d_tofc, sizeof tofc)) != cudaSuccess) return fail(cuda_fail(e, "cudaMalloc tof"));
+    if ((e = cudaMemcpy(h->d_tofc, tofc, sizeof tofc, cudaMemcpyHostToDevice)) != cudaSuccess)
         return fail(cuda_fail(e, "upload tof centres"));
     t.centers = h->d_tofc;
+    t.sorted = h->d_tofc + kMaxTofBins;
+    t.order = reinterpret_cast<const int *>(h->d_tofc + 2 * kMaxTofBins);
     if (desc->fp_type == 5) {
         if ((e = cudaMalloc(&h->d_imgT, h->n_img * sizeof(float))) != cudaSuccess)
             return fail(cuda_fail(e, "cudaMalloc type-5 image copy"));

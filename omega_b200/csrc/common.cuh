@@ -103,6 +103,12 @@ struct Tof {
     float sigma_coef;   // 1/sqrt(2 pi) / sigma
     float epps;
     const float *centers;
+    // sliding window of bins (tof.cuh)
+    const float *sorted;  // the centres in ascending order
+    const int *order;     // and which bin each one is
+    float k2, kv, kq;     // exponents per mm^2 (base 2) and series scale of the window's weights
+    int series;           // the weights' cosh series holds for every element
+    int window;           // bins a thread keeps (one of kTofWindows)
 };
 
 // Per-projection constants of the distance-driven backprojection: a

@@ -116,50 +116,58 @@ __device__ __forceinline__ float trilinear(const T *__restrict__ img, const Grid
     return fmaf(az, c1 - c0, c0);
 }
 
-// At most 80 registers (3 CTAs of 256 per SM): with the TOF weights' four
-// exponentials in flight per bin the forward projection otherwise takes 86
-// and falls to 2 CTAs (67.3 against 72.8 ms for 16 subsets x 15 bins).
-template <int NB, typename T>
-__global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof tof, float gf, float dL, const T *__restrict__ img,
-                            float *__restrict__ y) {
+// W: bins a thread keeps of a TOF measurement (tof.cuh), 0 without TOF.
+template <int W, typename T>
+__global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof tof, float gf, float dL,
+                                                         const T *__restrict__ img, float *__restrict__ y) {
     const bool pet = rs.modality != OMB_CT_PANEL;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rs.m_size; r += stride) {
-        float ax[NB];
-#pragma unroll
-        for (int to = 0; to < NB; ++to) ax[to] = 0.f;
         const Ray ray = load_ray(rs, r);
         March m;
-        float temp = 0.f;
-        if (march_setup(g, ray, dL, m)) {
-            temp = pet ? (1.f / m.L) * gf : 1.f;
-            const float ddsign = sgnf(m.D0);
-            float w[NB > 1 ? NB : 1];
+        if (!march_setup(g, ray, dL, m)) {
+            for (int to = 0; to < tof.nbins; ++to) y[r + to * rs.m_size] = 0.f;
+            continue;
+        }
+        const float temp = pet ? (1.f / m.L) * gf : 1.f;
+        auto sample = [&](float fi) {
+            return dL * trilinear(img, g, fmaf(fi, m.sx, m.cx), fmaf(fi, m.sy, m.cy), fmaf(fi, m.sz, m.cz));
+        };
+        if constexpr (W == 0) {
+            float ax = 0.f;
+            for (unsigned ii = 0; ii < m.n; ++ii) ax += sample((float)ii);
+            y[r] = ax * temp;
+        } else {
+            TofWindow<W> win;
+            win.begin(tof, sgnf(m.D0));
+            const float p0 = fmaf(0.5f * dL, win.moving, win.dir * m.D0), dp = dL * win.moving;
+            auto put = [&](int j, float v) { y[r + win.slot(tof, j) * rs.m_size] = v; };
             for (unsigned ii = 0; ii < m.n; ++ii) {
                 const float fi = (float)ii;
-                const float val =
-                    dL * trilinear(img, g, fmaf(fi, m.sx, m.cx), fmaf(fi, m.sy, m.cy), fmaf(fi, m.sz, m.cz));
-                if (NB == 1) {
-                    ax[0] += val;
-                } else {
-                    const float D = fmaf(-fi * dL, ddsign, m.D0);
-                    const float tsum = tof_weights<NB>(tof, ddsign, dL, D, w);
-                    const float dX = val / tsum;
-#pragma unroll
-                    for (int to = 0; to < NB; ++to) ax[to] = fmaf(w[to], dX, ax[to]);
+                const float val = sample(fi);
+                const float p = fmaf(fi, dp, p0);
+                while (p > win.th) {
+                    put(win.k, win.a[0] * temp);
+                    win.advance(tof, 0.f);
                 }
-            }
-        }
+                float w[W], sum;
+                const float dX = val * win.weights(tof, p, dL, w, sum);
 #pragma unroll
-        for (int to = 0; to < NB; ++to) y[r + to * rs.m_size] = ax[to] * temp;
+                for (int i = 0; i < W; ++i) win.a[i] = fmaf(w[i], dX, win.a[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+                if (win.k + i < tof.nbins) put(win.k + i, win.a[i] * temp);
+            for (int j = win.k + W; j < tof.nbins; ++j) put(j, 0.f);
+        }
     }
 }
 
 // Ray-driven PET backprojection.  FIXED: int64 fixed-point accumulators
 // (order independent, identical run to run); else float atomics.  y == NULL
 // backprojects ones; img == NULL (float mode) keeps only the sensitivity.
-template <int NB, bool SENS, bool FIXED>
-__global__ void k_interp_bp(Grid g, RaySet rs, Tof tof, float gf, float dL,
+template <int W, bool SENS, bool FIXED>
+__global__ void __launch_bounds__(kBlock) k_interp_bp(Grid g, RaySet rs, Tof tof, float gf, float dL,
                                                       const float *__restrict__ y, float *__restrict__ img,
                                                       float *__restrict__ sens, unsigned long long *__restrict__ acc,
                                                       unsigned long long *__restrict__ acc_s) {
@@ -170,20 +178,27 @@ __global__ void k_interp_bp(Grid g, RaySet rs, Tof tof, float gf, float dL,
     const double ivx = __ddiv_rn(1.0, (double)g.dx), ivy = __ddiv_rn(1.0, (double)g.dy),
                  ivz = __ddiv_rn(1.0, (double)g.dz);
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rs.m_size; r += stride) {
-        float ax[NB];
         bool any = SENS || y == nullptr;
-#pragma unroll
-        for (int to = 0; to < NB; ++to) {
-            ax[to] = y ? __ldg(y + r + to * rs.m_size) : 1.f;
-            any |= ax[to] != 0.f;
-        }
+        if (!any)
+            for (int to = 0; to < tof.nbins; ++to) any |= __ldg(y + r + to * rs.m_size) != 0.f;
         if (!any) continue;
         const Ray ray = load_ray(rs, r);
         March m;
         if (!march_setup(g, ray, dL, m)) continue;
         const float le = dL * ((1.f / m.L) * gf);
-        const float ddsign = sgnf(m.D0);
-        float w[NB > 1 ? NB : 1];
+        TofWindow<(W > 0 ? W : 2)> win;
+        float y1 = 0.f, p = 0.f;
+        auto get = [&](int j) { return y ? __ldg(y + r + win.slot(tof, j) * rs.m_size) : 1.f; };
+        if constexpr (W == 0) {
+            y1 = y ? __ldg(y + r) : 1.f;
+        } else {
+            win.begin(tof, sgnf(m.D0));
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+                if (i < tof.nbins) win.a[i] = get(i);
+            p = fmaf(0.5f * dL, win.moving, win.dir * m.D0);
+        }
+        const float p0 = p, dp = dL * win.moving;
         // TOF distance: advanced only after samples that land in the image (the
         // reference's loop skips its decrement together with the sample)
         unsigned kd = 0;
@@ -199,25 +214,22 @@ __global__ void k_interp_bp(Grid g, RaySet rs, Tof tof, float gf, float dL,
             const unsigned uy = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sy, __dmul_rn(vy, t)), by), ivy));
             const unsigned uz = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sz, __dmul_rn(vz, t)), bz), ivz));
             const unsigned ind = ux + uy * nx + uz * nxy;
-            float yax, val;
-            if (NB == 1) {
-                yax = ax[0] * le;
-                val = le;
-                if (isnan(le)) yax = 0.f;
-            } else {
-                const float D = fmaf(-(float)kd * dL, ddsign, m.D0);
-                const float tsum = tof_weights<NB>(tof, ddsign, dL, D, w);
-                const float dX = le / tsum;
-                yax = 0.f;
-                val = 0.f;
-#pragma unroll
-                for (int to = 0; to < NB; ++to) {
-                    const float a = dX * w[to];
-                    val += a;
-                    yax += a * ax[to];
-                }
-            }
             if (ind == 0u || ind >= ntot) continue;
+            float yax, val;
+            if constexpr (W == 0) {
+                yax = isnan(le) ? 0.f : y1 * le;
+                val = le;
+            } else {
+                p = fmaf((float)kd, dp, p0);
+                while (p > win.th) win.advance(tof, get(win.k + W));
+                float w[W], sum;
+                const float dX = le * win.weights(tof, p, dL, w, sum);
+                yax = 0.f;
+#pragma unroll
+                for (int i = 0; i < W; ++i) yax = fmaf(w[i], win.a[i], yax);
+                yax *= dX;
+                val = sum * dX;
+            }
             ++kd;
             if (FIXED) {
                 const long long q = (long long)((double)yax * kFixedScale);
@@ -309,14 +321,11 @@ __global__ void k_interp_ct_bp(Grid g, const BddProj *__restrict__ pj, int nr, i
     }
 }
 
-#define OMB_NB_CASES(X) \
-    X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
-
 int interp_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, float dL, const float *img,
                    const __nv_bfloat16 *img16, float *y, const Tuning &tn, cudaStream_t st) {
     if (rs.m_size <= 0) return OMB_OK;
     const unsigned grid = grid_for(rs.m_size, tn.siddon_blocks_per_sm);
-    switch (tof.nbins) {
+    switch (tof.nbins == 1 ? 0 : tof.window) {
 #define X(n)                                                                                    \
     case n:                                                                                     \
         if (img16)                                                                              \
@@ -324,7 +333,8 @@ int interp_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, fl
         else                                                                                    \
             k_interp_fp<n, float><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, img, y);            \
         break;
-        OMB_NB_CASES(X)
+        X(0)
+        OMB_TOF_WINDOWS(X)
 #undef X
         default:
             return set_error(OMB_ERR_UNSUPPORTED, "TOF bin count above 16 is not built");
@@ -333,19 +343,19 @@ int interp_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, fl
     return OMB_OK;
 }
 
-template <int NB>
+template <int W>
 static void bp_launch4(unsigned grid, const Grid &g, const RaySet &rs, const Tof &tof, float gf, float dL,
                        const float *y, float *img, float *sens, unsigned long long *acc, unsigned long long *acc_s,
                        cudaStream_t st) {
     if (acc) {
         if (acc_s)
-            k_interp_bp<NB, true, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
+            k_interp_bp<W, true, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
         else
-            k_interp_bp<NB, false, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
+            k_interp_bp<W, false, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
     } else if (sens) {
-        k_interp_bp<NB, true, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
+        k_interp_bp<W, true, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
     } else {
-        k_interp_bp<NB, false, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
+        k_interp_bp<W, false, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
     }
 }
 
@@ -356,9 +366,10 @@ int interp_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, f
     if ((uint64_t)g.nx * g.ny * g.nz >= (1ull << 32))
         return set_error(OMB_ERR_UNSUPPORTED, "type-4 backprojection needs fewer than 2^32 voxels");
     const unsigned grid = grid_for(rs.m_size, tn.siddon_blocks_per_sm);
-    switch (tof.nbins) {
+    switch (tof.nbins == 1 ? 0 : tof.window) {
 #define X(n) case n: bp_launch4<n>(grid, g, rs, tof, gf, dL, y, img, sens, acc, acc_s, st); break;
-        OMB_NB_CASES(X)
+        X(0)
+        OMB_TOF_WINDOWS(X)
 #undef X
         default:
             return set_error(OMB_ERR_UNSUPPORTED, "TOF bin count above 16 is not built");

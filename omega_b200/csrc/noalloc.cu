@@ -17,6 +17,7 @@
 #include <mutex>
 
 #include "kernels.h"
+#include "tof.cuh"
 
 namespace omb {
 
@@ -119,6 +120,8 @@ extern "C" int omb_backward_fixed64_noalloc(const omb_geometry_desc *desc, int32
     tof.sigma_inv = d.tof_bins > 1 ? 1.f / d.sigma_x : 0.f;
     tof.sigma_coef = 0.3989423f * tof.sigma_inv;
     tof.centers = d.tof_centers;
+    if (tof.nbins > 1)
+        tof_setup(tof, nullptr, nullptr, nullptr, fmaxf(d.dL, sqrtf(g.dx * g.dx + g.dy * g.dy + g.dz * g.dz)));
     RaySet rs{};
     rs.xy = d.xy;
     rs.z = d.z;

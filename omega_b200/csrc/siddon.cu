@@ -20,11 +20,12 @@ namespace omb {
 // SM) beats the spills it costs (measured: 30.6 -> 23.6 ms single-frame, 6.0
 // -> 3.9 ms for the interleaved 8-frame walk); the TOF variants keep their
 // registers (their weight arrays would spill hundreds of bytes).
-template <int NB, int FB, typename T, int K>
-__global__ void __launch_bounds__(kBlock, NB == 1 ? 4 : 1) k_siddon_fp(Grid g, RaySet rs, Tof tof, float gf,
-                                                      const T *__restrict__ img, int64_t img_stride,
-                                                      float *__restrict__ y, int64_t y_stride, int n_frames) {
+template <int FB, typename T, int K>
+__global__ void __launch_bounds__(kBlock, 4) k_siddon_fp(Grid g, RaySet rs, float gf, const T *__restrict__ img,
+                                                         int64_t img_stride, float *__restrict__ y, int64_t y_stride,
+                                                         int n_frames) {
     const bool pet = rs.modality != OMB_CT_PANEL;
+    const Tof tof{1, 0.f, 0.f, 0.f, nullptr};
     const int f0 = blockIdx.y * FB;
     const int nf = min(FB, n_frames - f0);
     img += f0 * img_stride;
@@ -33,29 +34,77 @@ __global__ void __launch_bounds__(kBlock, NB == 1 ? 4 : 1) k_siddon_fp(Grid g, R
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rs.m_size; r += stride) {
         const Ray ray = load_ray(rs, r);
         const float gfr = pet && (rs.w || rs.mu) ? gf * ray_correction(g, rs, ray, r) : gf;
-        float ax[NB * FB];
+        float ax[FB];
 #pragma unroll
-        for (int to = 0; to < NB * FB; ++to) ax[to] = 0.f;
+        for (int f = 0; f < FB; ++f) ax[f] = 0.f;
         float temp = 0.f;
-        const bool ok = siddon_walk<NB, K>(g, ray, pet, gfr, tof, temp,
-                                        [&](int64_t ind, float ele, const float *w, float tsum) {
-                                            if (NB == 1) {
+        const bool ok = siddon_walk<1, K>(g, ray, pet, gfr, tof, temp,
+                                          [&](int64_t ind, float ele, const float *, float) {
 #pragma unroll
-                                                for (int f = 0; f < FB; ++f)
-                                                    if (f < nf) ax[f] += ele * ld_img(img + f * img_stride + ind);
-                                            } else {
-                                                const float dX = ele * ld_img(img + ind) / tsum;
+                                              for (int f = 0; f < FB; ++f)
+                                                  if (f < nf) ax[f] += ele * ld_img(img + f * img_stride + ind);
+                                          });
 #pragma unroll
-                                                for (int to = 0; to < NB; ++to) ax[to] += w[to] * dX;
-                                            }
-                                        });
-        if (NB == 1) {
+        for (int f = 0; f < FB; ++f)
+            if (f < nf) y[f * y_stride + r] = ok ? ax[f] * temp : 0.f;
+    }
+}
+
+// TOF forward projection: the ray's walk hands every element to its window of
+// bins (tof.cuh); a bin is written when the window leaves it.
+template <int W, typename T>
+struct FpTof {
+    const Tof &tof;
+    const T *__restrict__ img;
+    float *__restrict__ y;   // the ray's bin 0; bins n_rays apart
+    int64_t n_rays;
+    float temp;
+    TofWindow<W> win;
+    __device__ __forceinline__ void begin(float ddsign) { win.begin(tof, ddsign); }
+    __device__ __forceinline__ void put(int j, float v) { y[win.slot(tof, j) * n_rays] = v; }
+    __device__ __forceinline__ void operator()(int64_t ind, float ele, float D, float full) {
+        const float v = ld_img(img + ind);
+        const float p = fmaf(0.5f * full, win.moving, win.dir * D);
+        while (p > win.th) {
+            put(win.k, win.a[0] * temp);
+            win.advance(tof, 0.f);
+        }
+        float w[W], sum;
+        float f = win.weights(tof, p, full, w, sum);
+        if (ele != full) {
+            // the end of a row: its own weights over the full voxel's sum
+            float part[W], s2;
+            const float total = sum;
+            win.weights(tof, fmaf(0.5f * ele, win.moving, win.dir * D), ele, part, s2);
+            f = tof.sigma_coef * (ele / 3.f) / fmaxf(total * (tof.sigma_coef * (full / 3.f)), tof.epps);
 #pragma unroll
-            for (int f = 0; f < FB; ++f)
-                if (f < nf) y[f * y_stride + r] = ok ? ax[f] * temp : 0.f;
+            for (int i = 0; i < W; ++i) w[i] = part[i];
+        }
+        const float dX = ele * v * f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) win.a[i] = fmaf(w[i], dX, win.a[i]);
+    }
+    __device__ __forceinline__ void finish() {
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            if (win.k + i < tof.nbins) put(win.k + i, win.a[i] * temp);
+        for (int j = win.k + W; j < tof.nbins; ++j) put(j, 0.f);
+    }
+};
+
+template <int W, typename T>
+__global__ void __launch_bounds__(kBlock) k_siddon_fp_tof(Grid g, RaySet rs, Tof tof, float gf,
+                                                          const T *__restrict__ img, float *__restrict__ y) {
+    const bool pet = rs.modality != OMB_CT_PANEL;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rs.m_size; r += stride) {
+        const Ray ray = load_ray(rs, r);
+        const float gfr = pet && (rs.w || rs.mu) ? gf * ray_correction(g, rs, ray, r) : gf;
+        FpTof<W, T> vis{tof, img, y + r, rs.m_size, 0.f};
+        if (siddon_walk<0>(g, ray, pet, gfr, tof, vis.temp, vis)) {
+            vis.finish();
         } else {
-#pragma unroll
-            for (int to = 0; to < NB; ++to) y[r + to * rs.m_size] = ok ? ax[to] * temp : 0.f;
+            for (int to = 0; to < tof.nbins; ++to) y[r + to * rs.m_size] = 0.f;
         }
     }
 }
@@ -192,112 +241,135 @@ __global__ void __launch_bounds__(kBlock) k_siddon_bp_ilv(Grid g, RaySet rs, flo
 
 // Backprojection with float atomics (rhs(), general_opencl_functions.h:1212-1275).
 // Frame batching as in the forward kernel: one walk, FB images updated.
-template <int NB, int FB, bool SENS>
-__global__ void __launch_bounds__(kBlock) k_siddon_bp(Grid g, RaySet rs, Tof tof, float gf,
-                                                      const float *__restrict__ y, int64_t y_stride,
-                                                      float *__restrict__ img, int64_t img_stride,
+template <int FB, bool SENS>
+__global__ void __launch_bounds__(kBlock) k_siddon_bp(Grid g, RaySet rs, float gf, const float *__restrict__ y,
+                                                      int64_t y_stride, float *__restrict__ img, int64_t img_stride,
                                                       float *__restrict__ sens, int n_frames) {
     const bool pet = rs.modality != OMB_CT_PANEL;
+    const Tof tof{1, 0.f, 0.f, 0.f, nullptr};
     const int f0 = blockIdx.y * FB;
     const int nf = min(FB, n_frames - f0);
     if (y) y += f0 * y_stride;
     if (img) img += f0 * img_stride;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rs.m_size; r += stride) {
-        float ax[NB * FB];
+        float ax[FB];
         bool any = SENS;
-        if (NB == 1) {
 #pragma unroll
-            for (int f = 0; f < FB; ++f) {
-                ax[f] = (y && f < nf) ? __ldg(y + f * y_stride + r) : 0.f;  // y == NULL: sensitivity only
-                any |= ax[f] != 0.f;
-            }
-        } else {
-#pragma unroll
-            for (int to = 0; to < NB; ++to) {
-                ax[to] = y ? __ldg(y + r + to * rs.m_size) : 0.f;
-                any |= ax[to] != 0.f;
-            }
+        for (int f = 0; f < FB; ++f) {
+            ax[f] = (y && f < nf) ? __ldg(y + f * y_stride + r) : 0.f;  // y == NULL: sensitivity only
+            any |= ax[f] != 0.f;
         }
         if (!any) continue;  // adds only zeros
         const Ray ray = load_ray(rs, r);
         const float gfr = pet && (rs.w || rs.mu) ? gf * ray_correction(g, rs, ray, r) : gf;
         float temp = 0.f;
-        siddon_walk<NB>(g, ray, pet, gfr, tof, temp, [&](int64_t ind, float ele, const float *w, float tsum) {
+        siddon_walk<1>(g, ray, pet, gfr, tof, temp, [&](int64_t ind, float ele, const float *, float) {
             const float le = ele * temp;
-            if (NB == 1) {
-                if (!isnan(le)) {
+            if (!isnan(le)) {
 #pragma unroll
-                    for (int f = 0; f < FB; ++f) {
-                        const float yax = ax[f] * le;
-                        if (f < nf && yax != 0.f) atomicAdd(img + f * img_stride + ind, yax);
-                    }
+                for (int f = 0; f < FB; ++f) {
+                    const float yax = ax[f] * le;
+                    if (f < nf && yax != 0.f) atomicAdd(img + f * img_stride + ind, yax);
                 }
-                if (SENS && le != 0.f) atomicAdd(sens + ind, le);
-            } else {
-                const float dX = le / tsum;
-                float yax = 0.f, val = 0.f;
-#pragma unroll
-                for (int to = 0; to < NB; ++to) {
-                    const float a = dX * w[to];
-                    val += a;
-                    yax += a * ax[to];
-                }
-                if (yax != 0.f) atomicAdd(img + ind, yax);
-                if (SENS && val != 0.f) atomicAdd(sens + ind, val);
             }
+            if (SENS && le != 0.f) atomicAdd(sens + ind, le);
         });
     }
 }
 
-// Backprojection into int64 fixed point: every contribution is rounded to an
-// integer on its own (toward zero, as OpenCL convert_long) and the integer
-// sums are order independent, so the result is identical run to run.
-// Semantics of the reference's -DATOMIC path (general_opencl_functions.h:1264-1272).
-template <int NB, bool SENS>
-__global__ void __launch_bounds__(kBlock) k_siddon_bp_fixed(Grid g, RaySet rs, Tof tof, float gf,
-                                                            const float *__restrict__ y,
+// Backprojection of one frame into int64 fixed point: every contribution is
+// rounded to an integer on its own (toward zero, as OpenCL convert_long) and
+// the integer sums are order independent, so the result is identical run to
+// run.  Semantics of the reference's -DATOMIC path
+// (general_opencl_functions.h:1264-1272).
+__device__ __forceinline__ void add_fixed(unsigned long long *acc, int64_t ind, float v) {
+    const long long q = (long long)((double)v * kFixedScale);
+    if (q != 0) atomicAdd(acc + ind, (unsigned long long)q);
+}
+
+template <bool SENS>
+__global__ void __launch_bounds__(kBlock) k_siddon_bp_fixed(Grid g, RaySet rs, float gf, const float *__restrict__ y,
                                                             unsigned long long *__restrict__ acc,
                                                             unsigned long long *__restrict__ acc_sens) {
     const bool pet = rs.modality != OMB_CT_PANEL;
+    const Tof tof{1, 0.f, 0.f, 0.f, nullptr};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rs.m_size; r += stride) {
-        float ax[NB];
-        bool any = SENS;
-#pragma unroll
-        for (int to = 0; to < NB; ++to) {
-            ax[to] = __ldg(y + r + to * rs.m_size);
-            any |= ax[to] != 0.f;
-        }
-        if (!any) continue;
+        const float ax = __ldg(y + r);
+        if (!SENS && ax == 0.f) continue;
         const Ray ray = load_ray(rs, r);
         const float gfr = pet && (rs.w || rs.mu) ? gf * ray_correction(g, rs, ray, r) : gf;
         float temp = 0.f;
-        siddon_walk<NB>(g, ray, pet, gfr, tof, temp, [&](int64_t ind, float ele, const float *w, float tsum) {
+        siddon_walk<1>(g, ray, pet, gfr, tof, temp, [&](int64_t ind, float ele, const float *, float) {
             const float le = ele * temp;
-            float yax, val;
-            if (NB == 1) {
-                yax = ax[0] * le;
-                val = le;
-                if (isnan(le)) yax = 0.f;
-            } else {
-                const float dX = le / tsum;
-                yax = 0.f;
-                val = 0.f;
-#pragma unroll
-                for (int to = 0; to < NB; ++to) {
-                    const float a = dX * w[to];
-                    val += a;
-                    yax += a * ax[to];
-                }
-            }
-            const long long q = (long long)((double)yax * kFixedScale);
-            if (q != 0) atomicAdd(acc + ind, (unsigned long long)q);
-            if (SENS) {
-                const long long qs = (long long)((double)val * kFixedScale);
-                if (qs != 0) atomicAdd(acc_sens + ind, (unsigned long long)qs);
-            }
+            add_fixed(acc, ind, isnan(le) ? 0.f : ax * le);
+            if (SENS) add_fixed(acc_sens, ind, le);
         });
+    }
+}
+
+// TOF backprojection, float (acc == NULL) or fixed point: a bin's measurement
+// is read when the ray's window of bins (tof.cuh) reaches it.  y == NULL (float
+// mode) backprojects only the sensitivity.
+template <int W, bool SENS, bool FIXED>
+struct BpTof {
+    const Tof &tof;
+    const float *__restrict__ y;
+    int64_t n_rays;
+    float *__restrict__ img, *__restrict__ sens;
+    unsigned long long *__restrict__ acc, *__restrict__ acc_sens;
+    float temp;
+    TofWindow<W> win;
+    __device__ __forceinline__ float get(int j) const { return y ? __ldg(y + win.slot(tof, j) * n_rays) : 0.f; }
+    __device__ __forceinline__ void begin(float ddsign) {
+        win.begin(tof, ddsign);
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            if (i < tof.nbins) win.a[i] = get(i);
+    }
+    __device__ __forceinline__ void operator()(int64_t ind, float ele, float D, float full) {
+        const float p = fmaf(0.5f * full, win.moving, win.dir * D);
+        while (p > win.th) win.advance(tof, get(win.k + W));
+        float w[W], sum;
+        float f = win.weights(tof, p, full, w, sum);
+        if (ele != full) {
+            const float total = sum;
+            win.weights(tof, fmaf(0.5f * ele, win.moving, win.dir * D), ele, w, sum);
+            f = tof.sigma_coef * (ele / 3.f) / fmaxf(total * (tof.sigma_coef * (full / 3.f)), tof.epps);
+        }
+        const float dX = ele * temp * f;
+        float back = 0.f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) back = fmaf(w[i], win.a[i], back);
+        const float yax = dX * back, val = dX * sum;
+        if (FIXED) {
+            add_fixed(acc, ind, yax);
+            if (SENS) add_fixed(acc_sens, ind, val);
+        } else {
+            if (yax != 0.f) atomicAdd(img + ind, yax);
+            if (SENS && val != 0.f) atomicAdd(sens + ind, val);
+        }
+    }
+};
+
+template <int W, bool SENS, bool FIXED>
+__global__ void __launch_bounds__(kBlock) k_siddon_bp_tof(Grid g, RaySet rs, Tof tof, float gf,
+                                                          const float *__restrict__ y, float *__restrict__ img,
+                                                          float *__restrict__ sens,
+                                                          unsigned long long *__restrict__ acc,
+                                                          unsigned long long *__restrict__ acc_sens) {
+    const bool pet = rs.modality != OMB_CT_PANEL;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rs.m_size; r += stride) {
+        bool any = SENS;
+        if (!SENS && y)
+            for (int to = 0; to < tof.nbins; ++to) any |= __ldg(y + r + to * rs.m_size) != 0.f;
+        if (!any) continue;  // adds only zeros
+        const Ray ray = load_ray(rs, r);
+        const float gfr = pet && (rs.w || rs.mu) ? gf * ray_correction(g, rs, ray, r) : gf;
+        BpTof<W, SENS, FIXED> vis{tof, y ? y + r : nullptr, rs.m_size, img, sens, acc, acc_sens, 0.f};
+        siddon_walk<0>(g, ray, pet, gfr, tof, vis.temp, vis);
     }
 }
 
@@ -339,53 +411,62 @@ __global__ void k_fixed_to_float(const unsigned long long *__restrict__ acc, flo
         out[i] = (float)((double)(long long)acc[i] * (1.0 / kFixedScale));
 }
 
-template <int NB, int FB, int K>
-static void fp_launch_k(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const Frames &fr, int per_sm,
-                        cudaStream_t st) {
+template <int FB, int K>
+static void fp_launch_k(const Grid &g, const RaySet &rs, float gf, const Frames &fr, int per_sm, cudaStream_t st) {
     dim3 grid(grid_for(rs.m_size, per_sm), (fr.n + FB - 1) / FB);
     if (fr.img_in16)
-        k_siddon_fp<NB, FB, __nv_bfloat16, K><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, fr.img_in16, fr.img_stride,
-                                                                       fr.meas_out, fr.meas_stride, fr.n);
+        k_siddon_fp<FB, __nv_bfloat16, K><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.img_in16, fr.img_stride, fr.meas_out,
+                                                                   fr.meas_stride, fr.n);
     else
-        k_siddon_fp<NB, FB, float, K><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, fr.img_in, fr.img_stride, fr.meas_out,
-                                                               fr.meas_stride, fr.n);
+        k_siddon_fp<FB, float, K><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.img_in, fr.img_stride, fr.meas_out,
+                                                           fr.meas_stride, fr.n);
 }
 
-// k: crossings taken per batched walk step (1, 2, 4; TOF walks take 1)
-template <int NB, int FB>
-static void fp_launch(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const Frames &fr, int per_sm, int k,
+// k: crossings taken per batched walk step (1, 2, 4)
+template <int FB>
+static void fp_launch(const Grid &g, const RaySet &rs, float gf, const Frames &fr, int per_sm, int k,
                       cudaStream_t st) {
-    if constexpr (NB == 1) {
-        if (k == 4) return fp_launch_k<NB, FB, 4>(g, rs, tof, gf, fr, per_sm, st);
-        if (k == 2) return fp_launch_k<NB, FB, 2>(g, rs, tof, gf, fr, per_sm, st);
-    }
-    fp_launch_k<NB, FB, 1>(g, rs, tof, gf, fr, per_sm, st);
+    if (k == 4) return fp_launch_k<FB, 4>(g, rs, gf, fr, per_sm, st);
+    if (k == 2) return fp_launch_k<FB, 2>(g, rs, gf, fr, per_sm, st);
+    fp_launch_k<FB, 1>(g, rs, gf, fr, per_sm, st);
 }
 
-template <int NB, int FB>
-static void bp_launch(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const Frames &fr, float *sens,
-                      int per_sm, cudaStream_t st) {
+template <int FB>
+static void bp_launch(const Grid &g, const RaySet &rs, float gf, const Frames &fr, float *sens, int per_sm,
+                      cudaStream_t st) {
     dim3 grid(grid_for(rs.m_size, per_sm), (fr.n + FB - 1) / FB);
     if (sens)
-        k_siddon_bp<NB, FB, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, fr.meas, fr.meas_stride, fr.img,
-                                                             fr.img_stride, sens, fr.n);
+        k_siddon_bp<FB, true><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, fr.img_stride, sens,
+                                                       fr.n);
     else
-        k_siddon_bp<NB, FB, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, fr.meas, fr.meas_stride, fr.img,
-                                                              fr.img_stride, nullptr, fr.n);
+        k_siddon_bp<FB, false><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, fr.img_stride,
+                                                        nullptr, fr.n);
 }
 
-template <int NB>
-static void bp_fixed_launch(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const float *y,
-                            unsigned long long *acc, unsigned long long *acc_sens, cudaStream_t st) {
-    const unsigned grid = grid_for(rs.m_size);
-    if (acc_sens)
-        k_siddon_bp_fixed<NB, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, acc, acc_sens);
+template <int W>
+static void fp_tof_launch(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const Frames &fr, int per_sm,
+                          cudaStream_t st) {
+    const unsigned grid = grid_for(rs.m_size, per_sm);
+    if (fr.img_in16)
+        k_siddon_fp_tof<W, __nv_bfloat16><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, fr.img_in16, fr.meas_out);
     else
-        k_siddon_bp_fixed<NB, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, acc, nullptr);
+        k_siddon_fp_tof<W, float><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, fr.img_in, fr.meas_out);
 }
 
-#define OMB_NB_CASES(X) \
-    X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
+template <int W>
+static void bp_tof_launch(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const float *y, float *img,
+                          float *sens, unsigned long long *acc, unsigned long long *acc_sens, int per_sm,
+                          cudaStream_t st) {
+    const unsigned grid = grid_for(rs.m_size, per_sm);
+    if (acc && acc_sens)
+        k_siddon_bp_tof<W, true, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
+    else if (acc)
+        k_siddon_bp_tof<W, false, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
+    else if (sens)
+        k_siddon_bp_tof<W, true, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
+    else
+        k_siddon_bp_tof<W, false, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
+}
 
 // Frames per walk for non-TOF batches (at most `most`).
 static int frames_per_walk(int n, int most) {
@@ -444,15 +525,15 @@ int siddon_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, co
         fp_ilv_launch<4>(g, rs, gf, fr, n_img, ps, k, st);
     } else if (tof.nbins == 1) {
         switch (frames_per_walk(fr.n, tn.siddon_frames)) {
-            case 8: fp_launch<1, 8>(g, rs, tof, gf, fr, ps, k, st); break;
-            case 4: fp_launch<1, 4>(g, rs, tof, gf, fr, ps, k, st); break;
-            case 2: fp_launch<1, 2>(g, rs, tof, gf, fr, ps, k, st); break;
-            default: fp_launch<1, 1>(g, rs, tof, gf, fr, ps, k, st); break;
+            case 8: fp_launch<8>(g, rs, gf, fr, ps, k, st); break;
+            case 4: fp_launch<4>(g, rs, gf, fr, ps, k, st); break;
+            case 2: fp_launch<2>(g, rs, gf, fr, ps, k, st); break;
+            default: fp_launch<1>(g, rs, gf, fr, ps, k, st); break;
         }
     } else {
-        switch (tof.nbins) {
-#define X(n) case n: fp_launch<n, 1>(g, rs, tof, gf, fr, ps, 1, st); break;
-            OMB_NB_CASES(X)
+        switch (tof.window) {
+#define X(n) case n: fp_tof_launch<n>(g, rs, tof, gf, fr, ps, st); break;
+            OMB_TOF_WINDOWS(X)
 #undef X
             default:
                 return set_error(OMB_ERR_UNSUPPORTED, "TOF bin count above 16 is not built");
@@ -478,15 +559,15 @@ int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, c
         if (e != OMB_OK) return e;
     } else if (tof.nbins == 1) {
         switch (frames_per_walk(fr.n, tn.siddon_frames)) {
-            case 8: bp_launch<1, 8>(g, rs, tof, gf, fr, sens, ps, st); break;
-            case 4: bp_launch<1, 4>(g, rs, tof, gf, fr, sens, ps, st); break;
-            case 2: bp_launch<1, 2>(g, rs, tof, gf, fr, sens, ps, st); break;
-            default: bp_launch<1, 1>(g, rs, tof, gf, fr, sens, ps, st); break;
+            case 8: bp_launch<8>(g, rs, gf, fr, sens, ps, st); break;
+            case 4: bp_launch<4>(g, rs, gf, fr, sens, ps, st); break;
+            case 2: bp_launch<2>(g, rs, gf, fr, sens, ps, st); break;
+            default: bp_launch<1>(g, rs, gf, fr, sens, ps, st); break;
         }
     } else {
-        switch (tof.nbins) {
-#define X(n) case n: bp_launch<n, 1>(g, rs, tof, gf, fr, sens, ps, st); break;
-            OMB_NB_CASES(X)
+        switch (tof.window) {
+#define X(n) case n: bp_tof_launch<n>(g, rs, tof, gf, fr.meas, fr.img, sens, nullptr, nullptr, ps, st); break;
+            OMB_TOF_WINDOWS(X)
 #undef X
             default:
                 return set_error(OMB_ERR_UNSUPPORTED, "TOF bin count above 16 is not built");
@@ -499,12 +580,27 @@ int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, c
 int siddon_backward_fixed(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const float *y,
                           unsigned long long *acc, unsigned long long *acc_sens, cudaStream_t st) {
     if (rs.m_size <= 0) return OMB_OK;
-    switch (tof.nbins) {
-#define X(n) case n: bp_fixed_launch<n>(g, rs, tof, gf, y, acc, acc_sens, st); break;
-        OMB_NB_CASES(X)
+    const unsigned grid = grid_for(rs.m_size);
+    if (tof.nbins == 1) {
+        if (acc_sens)
+            k_siddon_bp_fixed<true><<<grid, kBlock, 0, st>>>(g, rs, gf, y, acc, acc_sens);
+        else
+            k_siddon_bp_fixed<false><<<grid, kBlock, 0, st>>>(g, rs, gf, y, acc, nullptr);
+    } else {
+        // every bin in the window, in the given order: callers that hold the
+        // centres on the device only (omb_backward_fixed64_noalloc) cannot have
+        // them sorted, and both must give the same integers
+        Tof t = tof;
+        t.sorted = t.centers;
+        t.order = nullptr;
+        t.window = (t.nbins + 1) / 2 * 2;
+        switch (t.window) {
+#define X(n) case n: bp_tof_launch<n>(g, rs, t, gf, y, nullptr, nullptr, acc, acc_sens, 8, st); break;
+            OMB_TOF_WINDOWS(X)
 #undef X
-        default:
-            return set_error(OMB_ERR_UNSUPPORTED, "TOF bin count above 16 is not built");
+            default:
+                return set_error(OMB_ERR_UNSUPPORTED, "TOF bin count above 16 is not built");
+        }
     }
     OMB_LAUNCH_CHECK("siddon fixed-point backward launch");
     return OMB_OK;

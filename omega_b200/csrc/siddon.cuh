@@ -25,6 +25,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tof.cuh"
 
 namespace omb {
 
@@ -325,6 +326,11 @@ __device__ __forceinline__ float tof_weights(const Tof &tof, float ddsign, float
 // 0 at the batch's first (valid) voxel.  The visits and their order are those
 // of K = 1.
 //
+// NB = 0 leaves the TOF weights to the visitor, which is an object: begin(ddsign)
+// is called once before the first voxel, and vis(linear_voxel_index, length, D,
+// length the weights are normalised with) for every voxel, D the signed
+// distance of the element's start from the ray's middle.
+//
 // FULL_ROW: a ray along an image row visits every voxel of the row at full
 // voxel length (the row attenuation sum of the reference's CPU projector,
 // projector_functions.h:1193-1205) instead of the part between its end points.
@@ -402,26 +408,31 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
         // and would put the ray in the centre bin), and the normalisation
         // integrates a full voxel width.
         float D = 0.f, ddsign = 0.f;
-        if (NB > 1) {
+        if (NB != 1) {
             D = (float)((d_d2 * (double)nrow) / copysign(2.0, along_x ? diff.y : diff.x));
             ddsign = sgnf(D);
         }
+        if constexpr (NB == 0) vis.begin(ddsign);
         // FULL_ROW: from voxel 0 to the row's end
         for (int ii = FULL_ROW ? 0 : x1; ii <= (FULL_ROW ? nrow - 1 : x2); ++ii) {
-            if (FULL_ROW) {
+            if constexpr (FULL_ROW) {
                 vis(base + (int64_t)ii * stride, fd2, w, 1.f);
                 continue;
             }
             float d_in = fd2;
             if (x1 > 0 && ii == x1) d_in = fT1;
             else if (x2 < nrow - 1 && ii == x2) d_in = fT2;
-            float tsum = 1.f;
-            if (NB > 1) {
-                tsum = tof_weights<NB>(tof, ddsign, fd2, D, w);
-                if (d_in != fd2) tof_weights<NB>(tof, ddsign, d_in, D, w);
+            if constexpr (NB == 0) {
+                vis(base + (int64_t)ii * stride, d_in, D, fd2);
+            } else {
+                float tsum = 1.f;
+                if constexpr (NB > 1) {
+                    tsum = tof_weights<NB>(tof, ddsign, fd2, D, w);
+                    if (d_in != fd2) tof_weights<NB>(tof, ddsign, d_in, D, w);
+                }
+                vis(base + (int64_t)ii * stride, d_in, w, tsum);
             }
-            vis(base + (int64_t)ii * stride, d_in, w, tsum);
-            if (NB > 1) D -= fd2 * ddsign;
+            if (NB != 1) D -= fd2 * ddsign;
         }
         return true;
     }
@@ -452,11 +463,12 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
     if (skip) return false;
 
     float D = 0.f, ddsign = 0.f;
-    if (NB > 1) {
+    if (NB != 1) {
         const double a = diff.x * tcd, b = diff.y * tcd, c = diff.z * tcd;
         D = (float)(sqrt(a * a + b * b + c * c) - Ld / 2.0);
         ddsign = sgnf(D);
     }
+    if constexpr (NB == 0) vis.begin(ddsign);
     float tc = (float)tcd;
     float tx = ax.next(), ty = ay.next(), tz = az.next();
     if constexpr (K > 1) {
@@ -520,10 +532,14 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
             const bool pass = (t0 >= 0.f && t0 <= 1.f) || (tc >= 0.f && tc <= 1.f);
             const float ele = pass ? (fminf(t0, 1.f) - fmaxf(tc, 0.f)) * L : 0.f;
             tc = t0;
-            float tsum = 1.f;
-            if (NB > 1) tsum = tof_weights<NB>(tof, ddsign, ele, D, w);
-            vis(ind, ele, w, tsum);
-            if (NB > 1) D -= ele * ddsign;
+            if constexpr (NB == 0) {
+                vis(ind, ele, D, ele);
+            } else {
+                float tsum = 1.f;
+                if constexpr (NB > 1) tsum = tof_weights<NB>(tof, ddsign, ele, D, w);
+                vis(ind, ele, w, tsum);
+            }
+            if (NB != 1) D -= ele * ddsign;
             if (ti < 0 || ti >= g.nx || tj < 0 || tj >= g.ny || tk < 0 || tk >= g.nz) break;
         }
     }
