@@ -116,6 +116,42 @@ __device__ __forceinline__ float trilinear(const T *__restrict__ img, const Grid
     return fmaf(az, c1 - c0, c0);
 }
 
+// The same where all eight voxels lie inside the image (0 <= coordinate < size
+// - 1 on every axis): no clamps, and floor by adding 2^23 rounded down, whose
+// low bits are the index -- conversions and FRND share the special-function
+// pipe, six of them per sample.  CT forward + back at 301 x 218 x 90 rays, 170 x
+// 170 x 121: 4.46 -> 4.31 ms; 15-bin TOF pair 3.46 -> 3.25 ms.
+template <typename T>
+__device__ __forceinline__ float trilinear_inside(const T *__restrict__ img, int nx, int nxy, float x, float y,
+                                                  float z) {
+    const float big = 8388608.f;
+    const float tx = __fadd_rd(x, big), ty = __fadd_rd(y, big), tz = __fadd_rd(z, big);
+    const float ax = x - (tx - big), ay = y - (ty - big), az = z - (tz - big);
+    const int ix = __float_as_int(tx) & 0x7fffff, iy = __float_as_int(ty) & 0x7fffff,
+              iz = __float_as_int(tz) & 0x7fffff;
+    const T *p00 = img + ((int64_t)iz * nxy + (iy * nx + ix)), *p10 = p00 + nx, *p01 = p00 + nxy, *p11 = p10 + nxy;
+    const float v000 = ld_img(p00), v100 = ld_img(p00 + 1), v010 = ld_img(p10), v110 = ld_img(p10 + 1);
+    const float v001 = ld_img(p01), v101 = ld_img(p01 + 1), v011 = ld_img(p11), v111 = ld_img(p11 + 1);
+    const float c00 = fmaf(ax, v100 - v000, v000), c10 = fmaf(ax, v110 - v010, v010);
+    const float c01 = fmaf(ax, v101 - v001, v001), c11 = fmaf(ax, v111 - v011, v011);
+    const float c0 = fmaf(ay, c10 - c00, c00), c1 = fmaf(ay, c11 - c01, c01);
+    return fmaf(az, c1 - c0, c0);
+}
+
+// Samples [lo, hi] of a march that lie inside on one axis (c + n s in [0, size
+// - 1), with a margin far above the rounding of c + n s); intersected into lo, hi.
+__device__ __forceinline__ void inside_range(float c, float s, int size, float &lo, float &hi) {
+    const float a = 0.01f - c, b = (float)(size - 1) - 0.01f - c;
+    if (fabsf(s) < 1e-6f) {
+        // (a sample count times 1e-6 stays far inside one voxel)
+        if (!(a <= -0.5f && b >= 0.5f)) hi = -1.f;
+        return;
+    }
+    const float p = a / s, q = b / s;
+    lo = fmaxf(lo, ceilf(fminf(p, q)));
+    hi = fminf(hi, floorf(fmaxf(p, q)));
+}
+
 // W: bins a thread keeps of a TOF measurement (tof.cuh), 0 without TOF.
 template <int W, typename T>
 __global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof tof, float gf, float dL,
@@ -130,8 +166,17 @@ __global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof 
             continue;
         }
         const float temp = pet ? (1.f / m.L) * gf : 1.f;
+        // samples whose eight voxels are all in the image (all but the first
+        // and last few of a ray)
+        float in_lo = 0.f, in_hi = 3.4e38f;
+        inside_range(m.cx, m.sx, g.nx, in_lo, in_hi);
+        inside_range(m.cy, m.sy, g.ny, in_lo, in_hi);
+        inside_range(m.cz, m.sz, g.nz, in_lo, in_hi);
+        const int nxy = g.nx * g.ny;
         auto sample = [&](float fi) {
-            return dL * trilinear(img, g, fmaf(fi, m.sx, m.cx), fmaf(fi, m.sy, m.cy), fmaf(fi, m.sz, m.cz));
+            const float x = fmaf(fi, m.sx, m.cx), y = fmaf(fi, m.sy, m.cy), z = fmaf(fi, m.sz, m.cz);
+            return dL * (fi >= in_lo && fi <= in_hi ? trilinear_inside(img, g.nx, nxy, x, y, z)
+                                                    : trilinear(img, g, x, y, z));
         };
         if constexpr (W == 0) {
             float ax = 0.f;
