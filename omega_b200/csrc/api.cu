@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "scratch.cuh"
 #include "tof.cuh"
 
 namespace omb {
@@ -512,6 +513,7 @@ int omb_create(const omb_geometry_desc *desc, omb_handle **out) {
     h->desc.n_meas = nullptr;
     h->n_meas.assign(desc->n_meas, desc->n_meas + desc->n_subsets + 1);
     cudaGetDevice(&h->device);
+    scratch_hold(h->device);
     Grid &g = h->grid;
     g.nx = (int)desc->nx; g.ny = (int)desc->ny; g.nz = (int)desc->nz;
     g.dx = desc->dx; g.dy = desc->dy; g.dz = desc->dz;
@@ -634,6 +636,7 @@ int omb_destroy(omb_handle *h) {
     for (auto &m : h->sysmats) sysmat_free(m);
     cudaFree(h->d_ym);
     for (void *p : h->retired) cudaFree(p);
+    scratch_drop(h->device);
     if (prev != h->device) cudaSetDevice(prev);
     delete h;
     return OMB_OK;
@@ -737,7 +740,7 @@ int omb_backward(omb_handle *h, int32_t subset, const float *y, float *image, fl
             st = interp_backward(h->grid, rs, h->tof, h->desc.global_factor, h->desc.dL, y, nullptr, nullptr, acc,
                                  acc_s, h->tune, s);
         else
-            st = siddon_backward_fixed(h->grid, rs, h->tof, h->desc.global_factor, y, acc, acc_s, s);
+            st = siddon_backward_fixed(h->grid, rs, h->tof, h->desc.global_factor, y, acc, acc_s, true, s);
         if (st != OMB_OK) return st;
         st = fixed_to_float(acc, image, h->n_img, s);
         if (st == OMB_OK && sens) st = fixed_to_float(acc_s, sens, h->n_img, s);

@@ -216,9 +216,11 @@ __global__ void k_bdd_bp_ray(Grid g, const float *__restrict__ xy, const float *
     }
 }
 
-// y-fastest copy of an x-fastest volume (per z slice, a 2-D transpose).
-__global__ void k_transpose_xy(const float *__restrict__ in, float *__restrict__ out, int nx, int ny, int nz) {
-    __shared__ float tile[32][33];
+// y-fastest copy of an x-fastest volume (per z slice, a 2-D transpose).  ADD:
+// adds a y-fastest volume (nx and ny those of `in`) to an x-fastest one.
+template <typename T, bool ADD>
+__global__ void k_transpose_xy(const T *__restrict__ in, T *__restrict__ out, int nx, int ny, int nz) {
+    __shared__ T tile[32][33];
     const int z = blockIdx.z;
     const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32;
     const int64_t zo = (int64_t)z * nx * ny;
@@ -229,8 +231,34 @@ __global__ void k_transpose_xy(const float *__restrict__ in, float *__restrict__
     __syncthreads();
     for (int xx = threadIdx.y; xx < 32; xx += blockDim.y) {
         const int y = y0 + threadIdx.x, x = x0 + xx;
-        if (x < nx && y < ny) out[zo + y + (int64_t)x * ny] = tile[threadIdx.x][xx];
+        if (x < nx && y < ny) {
+            T &o = out[zo + y + (int64_t)x * ny];
+            if constexpr (ADD)
+                o += tile[threadIdx.x][xx];
+            else
+                o = tile[threadIdx.x][xx];
+        }
     }
+}
+
+template <typename T, bool ADD>
+static int launch_transpose(int nx, int ny, int nz, const T *in, T *out, cudaStream_t st) {
+    k_transpose_xy<T, ADD><<<dim3((nx + 31) / 32, (ny + 31) / 32, nz), dim3(32, 8), 0, st>>>(in, out, nx, ny, nz);
+    OMB_LAUNCH_CHECK("transpose launch");
+    return OMB_OK;
+}
+
+int transpose_xy(const Grid &g, const float *in, float *out, cudaStream_t st) {
+    return launch_transpose<float, false>(g.nx, g.ny, g.nz, in, out, st);
+}
+int transpose_xy(const Grid &g, const __nv_bfloat16 *in, __nv_bfloat16 *out, cudaStream_t st) {
+    return launch_transpose<__nv_bfloat16, false>(g.nx, g.ny, g.nz, in, out, st);
+}
+int add_transposed(const Grid &g, const float *in, float *out, cudaStream_t st) {
+    return launch_transpose<float, true>(g.ny, g.nx, g.nz, in, out, st);
+}
+int add_transposed(const Grid &g, const unsigned long long *in, unsigned long long *out, cudaStream_t st) {
+    return launch_transpose<unsigned long long, true>(g.ny, g.nx, g.nz, in, out, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -402,9 +430,8 @@ int bdd_forward(const Grid &g, const float *xy, const float *uv, int nr, int nc,
                 int64_t nproj, const float *img, float *imgT, float *y, const Tuning &tn, cudaStream_t st) {
     if (nproj <= 0) return OMB_OK;
     if (nproj > 65535) return set_error(OMB_ERR_UNSUPPORTED, "more than 65535 projections in one call");
-    dim3 tg((g.nx + 31) / 32, (g.ny + 31) / 32, g.nz);
-    k_transpose_xy<<<tg, dim3(32, 8), 0, st>>>(img, imgT, g.nx, g.ny, g.nz);
-    OMB_LAUNCH_CHECK("transpose launch");
+    const int tr = transpose_xy(g, img, imgT, st);
+    if (tr != OMB_OK) return tr;
     if (tn.bdd_fp_staged && (tn.bdd_fp_cols == 8 || tn.bdd_fp_cols == 16) && bdd_fp_tma_supported(g, img, imgT))
         return bdd_forward_tma(g, xy, uv, nr, nc, pitch_y, proj0, nproj, img, imgT, y, tn.bdd_fp_cols, st);
     switch (tn.bdd_fp_cols) {

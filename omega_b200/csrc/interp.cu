@@ -35,6 +35,7 @@
 //    FP64-built projective map as the type-5 backprojection instead of the
 //    FP32 plane intersection (identical in exact arithmetic).
 #include "kernels.h"
+#include "scratch.cuh"
 #include "siddon.cuh"
 
 namespace omb {
@@ -155,7 +156,8 @@ __device__ __forceinline__ void inside_range(float c, float s, int size, float &
 // W: bins a thread keeps of a TOF measurement (tof.cuh), 0 without TOF.
 template <int W, typename T>
 __global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof tof, float gf, float dL,
-                                                         const T *__restrict__ img, float *__restrict__ y) {
+                                                         const T *__restrict__ img, const T *__restrict__ imgT,
+                                                         float *__restrict__ y) {
     const bool pet = rs.modality != OMB_CT_PANEL;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rs.m_size; r += stride) {
@@ -166,17 +168,31 @@ __global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof 
             continue;
         }
         const float temp = pet ? (1.f / m.L) * gf : 1.f;
+        // rays along x read the y-fastest copy: x and y change places
+        Grid gr = g;
+        const T *im = img;
+        if (W == 0 && imgT && runs_along_x(ray.s, ray.d)) {
+            im = imgT;
+            gr.nx = g.ny;
+            gr.ny = g.nx;
+            float t = m.cx;
+            m.cx = m.cy;
+            m.cy = t;
+            t = m.sx;
+            m.sx = m.sy;
+            m.sy = t;
+        }
         // samples whose eight voxels are all in the image (all but the first
         // and last few of a ray)
         float in_lo = 0.f, in_hi = 3.4e38f;
-        inside_range(m.cx, m.sx, g.nx, in_lo, in_hi);
-        inside_range(m.cy, m.sy, g.ny, in_lo, in_hi);
-        inside_range(m.cz, m.sz, g.nz, in_lo, in_hi);
+        inside_range(m.cx, m.sx, gr.nx, in_lo, in_hi);
+        inside_range(m.cy, m.sy, gr.ny, in_lo, in_hi);
+        inside_range(m.cz, m.sz, gr.nz, in_lo, in_hi);
         const int nxy = g.nx * g.ny;
         auto sample = [&](float fi) {
             const float x = fmaf(fi, m.sx, m.cx), y = fmaf(fi, m.sy, m.cy), z = fmaf(fi, m.sz, m.cz);
-            return dL * (fi >= in_lo && fi <= in_hi ? trilinear_inside(img, g.nx, nxy, x, y, z)
-                                                    : trilinear(img, g, x, y, z));
+            return dL * (fi >= in_lo && fi <= in_hi ? trilinear_inside(im, gr.nx, nxy, x, y, z)
+                                                    : trilinear(im, gr, x, y, z));
         };
         if constexpr (W == 0) {
             float ax = 0.f;
@@ -214,10 +230,12 @@ __global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof 
 template <int W, bool SENS, bool FIXED>
 __global__ void __launch_bounds__(kBlock) k_interp_bp(Grid g, RaySet rs, Tof tof, float gf, float dL,
                                                       const float *__restrict__ y, float *__restrict__ img,
-                                                      float *__restrict__ sens, unsigned long long *__restrict__ acc,
+                                                      float *__restrict__ imgT, float *__restrict__ sens,
+                                                      unsigned long long *__restrict__ acc,
+                                                      unsigned long long *__restrict__ accT,
                                                       unsigned long long *__restrict__ acc_s) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const unsigned nx = (unsigned)g.nx, nxy = (unsigned)g.nx * (unsigned)g.ny;
+    const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny, nxy = nx * ny;
     const unsigned ntot = nxy * (unsigned)g.nz;
     const double bx = g.bx, by = g.by, bz = g.bz;
     const double ivx = __ddiv_rn(1.0, (double)g.dx), ivy = __ddiv_rn(1.0, (double)g.dy),
@@ -253,6 +271,9 @@ __global__ void __launch_bounds__(kBlock) k_interp_bp(Grid g, RaySet rs, Tof tof
         const double sx = ray.s.x, sy = ray.s.y, sz = ray.s.z;
         const double vx = __dsub_rn((double)ray.d.x, sx), vy = __dsub_rn((double)ray.d.y, sy),
                      vz = __dsub_rn((double)ray.d.z, sz);
+        // rays along x add to the y-fastest image; a sample off the grid's far
+        // faces in x or y lands on the x-fastest index it always had
+        const bool yfast = W == 0 && !SENS && (FIXED ? accT != nullptr : imgT != nullptr) && runs_along_x(ray.s, ray.d);
         for (unsigned ii = 0; ii < m.n; ++ii) {
             const double t = __dadd_rn(m.ts, __dmul_rn((double)ii, m.tstep));
             const unsigned ux = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sx, __dmul_rn(vx, t)), bx), ivx));
@@ -276,15 +297,17 @@ __global__ void __launch_bounds__(kBlock) k_interp_bp(Grid g, RaySet rs, Tof tof
                 val = sum * dX;
             }
             ++kd;
+            const bool turned = yfast && ux < nx && uy < ny;
+            const unsigned at = turned ? uy + ux * ny + uz * nxy : ind;
             if (FIXED) {
                 const long long q = (long long)((double)yax * kFixedScale);
-                if (q != 0) atomicAdd(acc + ind, (unsigned long long)q);
+                if (q != 0) atomicAdd((turned ? accT : acc) + at, (unsigned long long)q);
                 if (SENS) {
                     const long long qs = (long long)((double)val * kFixedScale);
                     if (qs != 0) atomicAdd(acc_s + ind, (unsigned long long)qs);
                 }
             } else {
-                if (img != nullptr && yax != 0.f) atomicAdd(img + ind, yax);
+                if (img != nullptr && yax != 0.f) atomicAdd((turned ? imgT : img) + at, yax);
                 if (SENS && val != 0.f) atomicAdd(sens + ind, val);
             }
         }
@@ -370,13 +393,22 @@ int interp_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, fl
                    const __nv_bfloat16 *img16, float *y, const Tuning &tn, cudaStream_t st) {
     if (rs.m_size <= 0) return OMB_OK;
     const unsigned grid = grid_for(rs.m_size, tn.siddon_blocks_per_sm);
+    const size_t vox = img16 ? sizeof(__nv_bfloat16) : sizeof(float);
+    const StreamScratch copy(tof.nbins == 1 && orient_pays(g, rs) ? (size_t)g.nx * g.ny * g.nz * vox : 0, st);
+    if (copy.p) {
+        const int e = img16 ? transpose_xy(g, img16, static_cast<__nv_bfloat16 *>(copy.p), st)
+                            : transpose_xy(g, img, static_cast<float *>(copy.p), st);
+        if (e != OMB_OK) return e;
+    }
     switch (tof.nbins == 1 ? 0 : tof.window) {
 #define X(n)                                                                                    \
     case n:                                                                                     \
         if (img16)                                                                              \
-            k_interp_fp<n, __nv_bfloat16><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, img16, y);  \
+            k_interp_fp<n, __nv_bfloat16><<<grid, kBlock, 0, st>>>(                             \
+                g, rs, tof, gf, dL, img16, static_cast<const __nv_bfloat16 *>(copy.p), y);      \
         else                                                                                    \
-            k_interp_fp<n, float><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, img, y);            \
+            k_interp_fp<n, float><<<grid, kBlock, 0, st>>>(                                     \
+                g, rs, tof, gf, dL, img, static_cast<const float *>(copy.p), y);                \
         break;
         X(0)
         OMB_TOF_WINDOWS(X)
@@ -390,17 +422,17 @@ int interp_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, fl
 
 template <int W>
 static void bp_launch4(unsigned grid, const Grid &g, const RaySet &rs, const Tof &tof, float gf, float dL,
-                       const float *y, float *img, float *sens, unsigned long long *acc, unsigned long long *acc_s,
-                       cudaStream_t st) {
+                       const float *y, float *img, float *imgT, float *sens, unsigned long long *acc,
+                       unsigned long long *accT, unsigned long long *acc_s, cudaStream_t st) {
     if (acc) {
         if (acc_s)
-            k_interp_bp<W, true, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
+            k_interp_bp<W, true, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
         else
-            k_interp_bp<W, false, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
+            k_interp_bp<W, false, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
     } else if (sens) {
-        k_interp_bp<W, true, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
+        k_interp_bp<W, true, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
     } else {
-        k_interp_bp<W, false, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, sens, acc, acc_s);
+        k_interp_bp<W, false, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
     }
 }
 
@@ -411,8 +443,14 @@ int interp_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, f
     if ((uint64_t)g.nx * g.ny * g.nz >= (1ull << 32))
         return set_error(OMB_ERR_UNSUPPORTED, "type-4 backprojection needs fewer than 2^32 voxels");
     const unsigned grid = grid_for(rs.m_size, tn.siddon_blocks_per_sm);
+    // rays along x add to a y-fastest image of their own, added to the result at the end
+    const size_t bytes = (size_t)g.nx * g.ny * g.nz * (acc ? sizeof(unsigned long long) : sizeof(float));
+    const StreamScratch along_x(!sens && !acc_s && (acc || img) && tof.nbins == 1 && orient_pays(g, rs) ? bytes : 0, st);
+    auto *accT = acc ? static_cast<unsigned long long *>(along_x.p) : nullptr;
+    auto *imgT = acc ? nullptr : static_cast<float *>(along_x.p);
+    if (along_x.p) OMB_CUDA_TRY(cudaMemsetAsync(along_x.p, 0, bytes, st));
     switch (tof.nbins == 1 ? 0 : tof.window) {
-#define X(n) case n: bp_launch4<n>(grid, g, rs, tof, gf, dL, y, img, sens, acc, acc_s, st); break;
+#define X(n) case n: bp_launch4<n>(grid, g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s, st); break;
         X(0)
         OMB_TOF_WINDOWS(X)
 #undef X
@@ -420,6 +458,8 @@ int interp_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, f
             return set_error(OMB_ERR_UNSUPPORTED, "TOF bin count above 16 is not built");
     }
     OMB_LAUNCH_CHECK("type-4 backward launch");
+    if (accT) return add_transposed(g, accT, acc, st);
+    if (imgT) return add_transposed(g, imgT, img, st);
     return OMB_OK;
 }
 

@@ -9,8 +9,14 @@ int siddon_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, co
                    cudaStream_t st);
 int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const Frames &fr, float *sens,
                     const Tuning &tn, cudaStream_t st);
+// may_allocate: the call may take scratch memory
 int siddon_backward_fixed(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const float *y,
-                          unsigned long long *acc, unsigned long long *acc_sens, cudaStream_t st);
+                          unsigned long long *acc, unsigned long long *acc_sens, bool may_allocate, cudaStream_t st);
+// y-fastest copy of an image, and the sum of one into an image (oriented images, common.cuh)
+int transpose_xy(const Grid &g, const float *in, float *out, cudaStream_t st);
+int transpose_xy(const Grid &g, const __nv_bfloat16 *in, __nv_bfloat16 *out, cudaStream_t st);
+int add_transposed(const Grid &g, const float *in, float *out, cudaStream_t st);
+int add_transposed(const Grid &g, const unsigned long long *in, unsigned long long *out, cudaStream_t st);
 int siddon_count(const Grid &g, const RaySet &rs, const Tof &tof, unsigned long long *total, cudaStream_t st);
 int fixed_to_float(const unsigned long long *acc, float *out, int64_t n, cudaStream_t st);
 

@@ -149,7 +149,7 @@ extern "C" int omb_backward_fixed64_noalloc(const omb_geometry_desc *desc, int32
     unsigned long long *acc_s = sens ? acc + n : nullptr;
     // the array keeps the previous call's sums: clear the part this call uses
     OMB_CUDA_TRY(cudaMemsetAsync(acc, 0, (sens ? 2 : 1) * n * sizeof(unsigned long long), s));
-    st = siddon_backward_fixed(g, rs, tof, d.global_factor, y, acc, acc_s, s);
+    st = siddon_backward_fixed(g, rs, tof, d.global_factor, y, acc, acc_s, false, s);
     if (st != OMB_OK) return st;
     st = fixed_to_float(acc, image, n, s);
     if (st == OMB_OK && sens) st = fixed_to_float(acc_s, sens, n, s);

@@ -7,6 +7,7 @@
 // cache (L2-resident for every image this path sees: 256 KiB-80 MiB).
 #include "siddon.cuh"
 #include "kernels.h"
+#include "scratch.cuh"
 
 namespace omb {
 
@@ -22,8 +23,8 @@ namespace omb {
 // registers (their weight arrays would spill hundreds of bytes).
 template <int FB, typename T, int K>
 __global__ void __launch_bounds__(kBlock, 4) k_siddon_fp(Grid g, RaySet rs, float gf, const T *__restrict__ img,
-                                                         int64_t img_stride, float *__restrict__ y, int64_t y_stride,
-                                                         int n_frames) {
+                                                         const T *__restrict__ imgT, int64_t img_stride,
+                                                         float *__restrict__ y, int64_t y_stride, int n_frames) {
     const bool pet = rs.modality != OMB_CT_PANEL;
     const Tof tof{1, 0.f, 0.f, 0.f, nullptr};
     const int f0 = blockIdx.y * FB;
@@ -38,12 +39,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_siddon_fp(Grid g, RaySet rs, floa
 #pragma unroll
         for (int f = 0; f < FB; ++f) ax[f] = 0.f;
         float temp = 0.f;
+        const bool yfast = FB == 1 && imgT && runs_along_x(ray.s, ray.d);
+        const T *im = yfast ? imgT : img;
         const bool ok = siddon_walk<1, K>(g, ray, pet, gfr, tof, temp,
                                           [&](int64_t ind, float ele, const float *, float) {
 #pragma unroll
                                               for (int f = 0; f < FB; ++f)
-                                                  if (f < nf) ax[f] += ele * ld_img(img + f * img_stride + ind);
-                                          });
+                                                  if (f < nf) ax[f] += ele * ld_img(im + f * img_stride + ind);
+                                          }, yfast);
 #pragma unroll
         for (int f = 0; f < FB; ++f)
             if (f < nf) y[f * y_stride + r] = ok ? ax[f] * temp : 0.f;
@@ -243,7 +246,8 @@ __global__ void __launch_bounds__(kBlock) k_siddon_bp_ilv(Grid g, RaySet rs, flo
 // Frame batching as in the forward kernel: one walk, FB images updated.
 template <int FB, bool SENS>
 __global__ void __launch_bounds__(kBlock) k_siddon_bp(Grid g, RaySet rs, float gf, const float *__restrict__ y,
-                                                      int64_t y_stride, float *__restrict__ img, int64_t img_stride,
+                                                      int64_t y_stride, float *__restrict__ img,
+                                                      float *__restrict__ imgT, int64_t img_stride,
                                                       float *__restrict__ sens, int n_frames) {
     const bool pet = rs.modality != OMB_CT_PANEL;
     const Tof tof{1, 0.f, 0.f, 0.f, nullptr};
@@ -264,17 +268,19 @@ __global__ void __launch_bounds__(kBlock) k_siddon_bp(Grid g, RaySet rs, float g
         const Ray ray = load_ray(rs, r);
         const float gfr = pet && (rs.w || rs.mu) ? gf * ray_correction(g, rs, ray, r) : gf;
         float temp = 0.f;
+        const bool yfast = FB == 1 && !SENS && imgT && runs_along_x(ray.s, ray.d);
+        float *im = yfast ? imgT : img;
         siddon_walk<1>(g, ray, pet, gfr, tof, temp, [&](int64_t ind, float ele, const float *, float) {
             const float le = ele * temp;
             if (!isnan(le)) {
 #pragma unroll
                 for (int f = 0; f < FB; ++f) {
                     const float yax = ax[f] * le;
-                    if (f < nf && yax != 0.f) atomicAdd(img + f * img_stride + ind, yax);
+                    if (f < nf && yax != 0.f) atomicAdd(im + f * img_stride + ind, yax);
                 }
             }
             if (SENS && le != 0.f) atomicAdd(sens + ind, le);
-        });
+        }, yfast);
     }
 }
 
@@ -291,6 +297,7 @@ __device__ __forceinline__ void add_fixed(unsigned long long *acc, int64_t ind, 
 template <bool SENS>
 __global__ void __launch_bounds__(kBlock) k_siddon_bp_fixed(Grid g, RaySet rs, float gf, const float *__restrict__ y,
                                                             unsigned long long *__restrict__ acc,
+                                                            unsigned long long *__restrict__ accT,
                                                             unsigned long long *__restrict__ acc_sens) {
     const bool pet = rs.modality != OMB_CT_PANEL;
     const Tof tof{1, 0.f, 0.f, 0.f, nullptr};
@@ -301,11 +308,13 @@ __global__ void __launch_bounds__(kBlock) k_siddon_bp_fixed(Grid g, RaySet rs, f
         const Ray ray = load_ray(rs, r);
         const float gfr = pet && (rs.w || rs.mu) ? gf * ray_correction(g, rs, ray, r) : gf;
         float temp = 0.f;
+        const bool yfast = !SENS && accT && runs_along_x(ray.s, ray.d);
+        unsigned long long *to = yfast ? accT : acc;
         siddon_walk<1>(g, ray, pet, gfr, tof, temp, [&](int64_t ind, float ele, const float *, float) {
             const float le = ele * temp;
-            add_fixed(acc, ind, isnan(le) ? 0.f : ax * le);
+            add_fixed(to, ind, isnan(le) ? 0.f : ax * le);
             if (SENS) add_fixed(acc_sens, ind, le);
-        });
+        }, yfast);
     }
 }
 
@@ -412,34 +421,36 @@ __global__ void k_fixed_to_float(const unsigned long long *__restrict__ acc, flo
 }
 
 template <int FB, int K>
-static void fp_launch_k(const Grid &g, const RaySet &rs, float gf, const Frames &fr, int per_sm, cudaStream_t st) {
+static void fp_launch_k(const Grid &g, const RaySet &rs, float gf, const Frames &fr, const void *imgT, int per_sm,
+                        cudaStream_t st) {
     dim3 grid(grid_for(rs.m_size, per_sm), (fr.n + FB - 1) / FB);
     if (fr.img_in16)
-        k_siddon_fp<FB, __nv_bfloat16, K><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.img_in16, fr.img_stride, fr.meas_out,
-                                                                   fr.meas_stride, fr.n);
+        k_siddon_fp<FB, __nv_bfloat16, K><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.img_in16,
+                                                                   static_cast<const __nv_bfloat16 *>(imgT), fr.img_stride,
+                                                                   fr.meas_out, fr.meas_stride, fr.n);
     else
-        k_siddon_fp<FB, float, K><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.img_in, fr.img_stride, fr.meas_out,
-                                                           fr.meas_stride, fr.n);
+        k_siddon_fp<FB, float, K><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.img_in, static_cast<const float *>(imgT),
+                                                           fr.img_stride, fr.meas_out, fr.meas_stride, fr.n);
 }
 
 // k: crossings taken per batched walk step (1, 2, 4)
 template <int FB>
-static void fp_launch(const Grid &g, const RaySet &rs, float gf, const Frames &fr, int per_sm, int k,
-                      cudaStream_t st) {
-    if (k == 4) return fp_launch_k<FB, 4>(g, rs, gf, fr, per_sm, st);
-    if (k == 2) return fp_launch_k<FB, 2>(g, rs, gf, fr, per_sm, st);
-    fp_launch_k<FB, 1>(g, rs, gf, fr, per_sm, st);
+static void fp_launch(const Grid &g, const RaySet &rs, float gf, const Frames &fr, const void *imgT, int per_sm,
+                      int k, cudaStream_t st) {
+    if (k == 4) return fp_launch_k<FB, 4>(g, rs, gf, fr, imgT, per_sm, st);
+    if (k == 2) return fp_launch_k<FB, 2>(g, rs, gf, fr, imgT, per_sm, st);
+    fp_launch_k<FB, 1>(g, rs, gf, fr, imgT, per_sm, st);
 }
 
 template <int FB>
-static void bp_launch(const Grid &g, const RaySet &rs, float gf, const Frames &fr, float *sens, int per_sm,
-                      cudaStream_t st) {
+static void bp_launch(const Grid &g, const RaySet &rs, float gf, const Frames &fr, float *imgT, float *sens,
+                      int per_sm, cudaStream_t st) {
     dim3 grid(grid_for(rs.m_size, per_sm), (fr.n + FB - 1) / FB);
     if (sens)
-        k_siddon_bp<FB, true><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, fr.img_stride, sens,
-                                                       fr.n);
+        k_siddon_bp<FB, true><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, nullptr, fr.img_stride,
+                                                       sens, fr.n);
     else
-        k_siddon_bp<FB, false><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, fr.img_stride,
+        k_siddon_bp<FB, false><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, imgT, fr.img_stride,
                                                         nullptr, fr.n);
 }
 
@@ -519,16 +530,24 @@ int siddon_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, co
     const int64_t n_img = (int64_t)g.nx * g.ny * g.nz;
     const int ilv = interleaved_frames(tof, fr, tn, n_img);
     const int k = tn.siddon_fp_steps;
+    // the y-fastest copy of a single image
+    const size_t vox = fr.img_in16 ? sizeof(__nv_bfloat16) : sizeof(float);
+    const StreamScratch copy(!ilv && fr.n == 1 && tof.nbins == 1 && orient_pays(g, rs) ? n_img * vox : 0, st);
+    if (copy.p) {
+        const int e = fr.img_in16 ? transpose_xy(g, fr.img_in16, static_cast<__nv_bfloat16 *>(copy.p), st)
+                                  : transpose_xy(g, fr.img_in, static_cast<float *>(copy.p), st);
+        if (e != OMB_OK) return e;
+    }
     if (ilv == 8) {
         fp_ilv_launch<8>(g, rs, gf, fr, n_img, ps, k, st);
     } else if (ilv == 4) {
         fp_ilv_launch<4>(g, rs, gf, fr, n_img, ps, k, st);
     } else if (tof.nbins == 1) {
         switch (frames_per_walk(fr.n, tn.siddon_frames)) {
-            case 8: fp_launch<8>(g, rs, gf, fr, ps, k, st); break;
-            case 4: fp_launch<4>(g, rs, gf, fr, ps, k, st); break;
-            case 2: fp_launch<2>(g, rs, gf, fr, ps, k, st); break;
-            default: fp_launch<1>(g, rs, gf, fr, ps, k, st); break;
+            case 8: fp_launch<8>(g, rs, gf, fr, nullptr, ps, k, st); break;
+            case 4: fp_launch<4>(g, rs, gf, fr, nullptr, ps, k, st); break;
+            case 2: fp_launch<2>(g, rs, gf, fr, nullptr, ps, k, st); break;
+            default: fp_launch<1>(g, rs, gf, fr, copy.p, ps, k, st); break;
         }
     } else {
         switch (tof.window) {
@@ -551,6 +570,11 @@ int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, c
     const int64_t n_img = (int64_t)g.nx * g.ny * g.nz;
     // the interleaved kernels write every voxel of every frame (no sensitivity)
     const int ilv = sens || !fr.meas || !fr.img ? 0 : interleaved_frames(tof, fr, tn, n_img);
+    // rays along x add to a y-fastest image of their own, added to the result at the end
+    const bool turn = !ilv && !sens && fr.n == 1 && tof.nbins == 1 && fr.meas && fr.img && orient_pays(g, rs);
+    const StreamScratch along_x(turn ? n_img * sizeof(float) : 0, st);
+    float *imgT = static_cast<float *>(along_x.p);
+    if (imgT) OMB_CUDA_TRY(cudaMemsetAsync(imgT, 0, n_img * sizeof(float), st));
     if (ilv == 8) {
         const int e = bp_ilv_launch<8>(g, rs, gf, fr, n_img, ps, st);
         if (e != OMB_OK) return e;
@@ -559,10 +583,10 @@ int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, c
         if (e != OMB_OK) return e;
     } else if (tof.nbins == 1) {
         switch (frames_per_walk(fr.n, tn.siddon_frames)) {
-            case 8: bp_launch<8>(g, rs, gf, fr, sens, ps, st); break;
-            case 4: bp_launch<4>(g, rs, gf, fr, sens, ps, st); break;
-            case 2: bp_launch<2>(g, rs, gf, fr, sens, ps, st); break;
-            default: bp_launch<1>(g, rs, gf, fr, sens, ps, st); break;
+            case 8: bp_launch<8>(g, rs, gf, fr, nullptr, sens, ps, st); break;
+            case 4: bp_launch<4>(g, rs, gf, fr, nullptr, sens, ps, st); break;
+            case 2: bp_launch<2>(g, rs, gf, fr, nullptr, sens, ps, st); break;
+            default: bp_launch<1>(g, rs, gf, fr, imgT, sens, ps, st); break;
         }
     } else {
         switch (tof.window) {
@@ -574,18 +598,22 @@ int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, c
         }
     }
     OMB_LAUNCH_CHECK("siddon backward launch");
-    return OMB_OK;
+    return imgT ? add_transposed(g, imgT, fr.img, st) : OMB_OK;
 }
 
 int siddon_backward_fixed(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const float *y,
-                          unsigned long long *acc, unsigned long long *acc_sens, cudaStream_t st) {
+                          unsigned long long *acc, unsigned long long *acc_sens, bool may_allocate, cudaStream_t st) {
     if (rs.m_size <= 0) return OMB_OK;
+    const size_t bytes = (size_t)g.nx * g.ny * g.nz * sizeof(unsigned long long);
+    const StreamScratch along_x(may_allocate && !acc_sens && tof.nbins == 1 && orient_pays(g, rs) ? bytes : 0, st);
+    auto *accT = static_cast<unsigned long long *>(along_x.p);
+    if (accT) OMB_CUDA_TRY(cudaMemsetAsync(accT, 0, bytes, st));
     const unsigned grid = grid_for(rs.m_size);
     if (tof.nbins == 1) {
         if (acc_sens)
-            k_siddon_bp_fixed<true><<<grid, kBlock, 0, st>>>(g, rs, gf, y, acc, acc_sens);
+            k_siddon_bp_fixed<true><<<grid, kBlock, 0, st>>>(g, rs, gf, y, acc, nullptr, acc_sens);
         else
-            k_siddon_bp_fixed<false><<<grid, kBlock, 0, st>>>(g, rs, gf, y, acc, nullptr);
+            k_siddon_bp_fixed<false><<<grid, kBlock, 0, st>>>(g, rs, gf, y, acc, accT, nullptr);
     } else {
         // every bin in the window, in the given order: callers that hold the
         // centres on the device only (omb_backward_fixed64_noalloc) cannot have
@@ -603,7 +631,7 @@ int siddon_backward_fixed(const Grid &g, const RaySet &rs, const Tof &tof, float
         }
     }
     OMB_LAUNCH_CHECK("siddon fixed-point backward launch");
-    return OMB_OK;
+    return accT ? add_transposed(g, accT, acc, st) : OMB_OK;
 }
 
 int fixed_to_float(const unsigned long long *acc, float *out, int64_t n, cudaStream_t st) {

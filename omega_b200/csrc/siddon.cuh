@@ -335,12 +335,14 @@ __device__ __forceinline__ float tof_weights(const Tof &tof, float ddsign, float
 // length the weights are normalised with) for every voxel, D the signed
 // distance of the element's start from the ray's middle.
 //
+// yfast: linear voxel indices of the y-fastest copy (oriented images).
+//
 // FULL_ROW: a ray along an image row visits every voxel of the row at full
 // voxel length (the row attenuation sum of the reference's CPU projector,
 // projector_functions.h:1193-1205) instead of the part between its end points.
 template <int NB, int K = 1, bool FULL_ROW = false, class Visit>
 __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool pet, float global_factor,
-                                            const Tof &tof, float &temp, Visit &&vis) {
+                                            const Tof &tof, float &temp, Visit &&vis, bool yfast = false) {
     // Set-up in FP64 (end points are FP32, so their differences are exact);
     // the per-voxel walk below runs in FP32.
     const D3 s{ray.s.x, ray.s.y, ray.s.z}, d{ray.d.x, ray.d.y, ray.d.z};
@@ -352,6 +354,7 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
     const float L = (float)Ld;
     temp = pet ? (float)(1.0 / Ld) * global_factor : 1.f;
     const int64_t nxy = (int64_t)g.nx * g.ny;
+    const int stx = yfast ? g.ny : 1, sty = yfast ? 1 : g.nx;
     float w[NB > 1 ? NB : 1];
     const double bx = g.bx, by = g.by, bz = g.bz, dxg = g.dx, dyg = g.dy, dzg = g.dz;
     const double mx = g.mx, my = g.my, mz = g.mz;
@@ -402,8 +405,8 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
         }
         const int row = perpendicular_start(d_b, dd, d_db, n0);
         // voxel (i, j, k): along x -> (ii, row, tk); along y -> (row, ii, tk)
-        const int64_t base = (int64_t)tk * nxy + (along_x ? (int64_t)row * g.nx : (int64_t)row);
-        const int64_t stride = along_x ? 1 : g.nx;
+        const int64_t base = (int64_t)tk * nxy + (int64_t)row * (along_x ? sty : stx);
+        const int64_t stride = along_x ? stx : sty;
         const float fd2 = (float)d_d2, fT1 = (float)dT1, fT2 = (float)dT2;
         // TOF along a row: the reference CPU projector's form
         // (projector_functions.h:1617-1685): D starts at +-half the row length
@@ -486,8 +489,8 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
     const float te = fminf(fminf(ax.leave(ti, g.nx), ay.leave(tj, g.ny)), az.leave(tk, g.nz));
     // both end points outside the grid (every scanner): no clamp to [0, 1]
     const bool through = tc >= 0.f && te <= 1.f;
-    int64_t ind = (int64_t)tj * g.nx + ti + (int64_t)tk * nxy;
-    const int dxi = ax.u, dyi = ay.u * g.nx;
+    int64_t ind = (int64_t)tj * sty + (int64_t)ti * stx + (int64_t)tk * nxy;
+    const int dxi = ax.u * stx, dyi = ay.u * sty;
     const int64_t dzi = az.u * nxy;
     auto step = [&](float &ele) {
         const bool z = tz < ty && tz < tx, y = !z && ty < tx;
