@@ -523,6 +523,13 @@ int omb_create(const omb_geometry_desc *desc, omb_handle **out) {
     g.my = desc->by + (float)desc->ny * desc->dy;
     g.mz = desc->bz + (float)desc->nz * desc->dz;
     h->n_img = (int64_t)desc->nx * desc->ny * desc->nz;
+    // Staged type-5 backprojection (bdd_bp_tma_supported): runs of 16 voxels
+    // share a footprint and a view's set-up among twice as many as 8 (90 views
+    // of 512 x 512, 256^3: 3.61 -> 2.94 ms) where the CTAs (32 x 4 columns of
+    // voxels) still fill every SM.
+    if (desc->bp_type == 5 && desc->n_rows_d % 4 == 0 && desc->nz >= 16 &&
+        (int64_t)((desc->nx + 31) / 32) * ((desc->ny + 3) / 4) * (desc->nz / 16) >= 5 * (int64_t)num_sms())
+        h->tune.bdd_bp_z = 16;
     Tof &t = h->tof;
     t.nbins = desc->tof_bins;
     t.epps = desc->epps;
