@@ -1,22 +1,35 @@
 // 3x3x3 convolution of the learned warm start on the 5th-generation tensor
 // cores: tcgen05.mma (kind::f16, BF16 operands, FP32 accumulator in tensor
-// memory), issued by one thread per CTA.
+// memory), its input staged once per block and read shifted by every tap.
 //
-// Implicit GEMM: a CTA computes D[128 voxels][COUT] = sum over 27 taps and
-// CIN/16 channel chunks of A[128][16] x B[16][COUT], A the tap-shifted input
-// rows (zero outside the volume), B the weights W[tap][co][ci].  Both
-// operands are staged in shared memory in the canonical K-major layout
-// without swizzle (core matrices of 8 rows x 16 bytes; the two 8-element K
-// halves 128 bytes apart, 8-row groups 256 bytes apart), double-buffered: the
-// CTA fills stage s^1 while the tensor core reads stage s, and
-// tcgen05.commit signals an mbarrier when a stage may be refilled.  The
-// epilogue reads the accumulator with tcgen05.ld (warp w owns TMEM lanes
-// 32w..32w+31 = voxels 32w..), adds the bias, applies the ReLU or the mask
-// and stores BF16.  Every mbarrier wait is bounded; on a timeout the CTA
-// raises the error flag read by omb_unet_take_error().  The weight gradient
-// (k_conv3d_wgrad_tc, below) runs on the same instructions with the voxels
-// as the reduction dimension.
+// A CTA computes a block of TX x TY x TZ voxels for up to 48 output channels.
+// Input planes (16 channels of a (TX+2) x (TY+2) halo at one z, zeros outside
+// the volume) stream through a ring of shared-memory stages, each loaded once
+// by three warps with 16-byte cp.async.  (TMA boxes would need an inner extent
+// of 16 bytes for this layout and then move about 3 bytes a clock.)  A stage holds 16-byte
+// rows (8 channels of a voxel) in voxel order, which is the canonical K-major
+// layout without swizzle with 8-row groups 128 bytes apart, so the operand of
+// a tap is the same rows at another start address: nothing is copied per tap.
+// The weights of all taps stay in shared memory, the three dz taps of one
+// (dy, dx) side by side: one instruction of N = 3 cout columns adds an input
+// plane to the three output planes it belongs to, whose accumulators are
+// neighbouring tensor-memory columns.  That reads A nine times per plane
+// instead of 27 (with N = 16 an instruction is bound by its 4 KB of A).
+// M = 128 rows are a line of voxels (TX = 128), else 128 consecutive positions
+// of the staged plane, whose halo columns are computed and not stored.
+// Warps: 0 issues instructions, 1-3 load, 4-7 store results.  Before this a CTA
+// staged 27 tap-shifted copies of 128 voxels through registers, one
+// instruction per pair of barriers: 32 -> 32 channels at 62 x 58 x 31 x 4 took
+// 197 us, now 89.
+//
+// Every wait is bounded; on a timeout the CTA raises the error flag read by
+// omb_unet_take_error(), waits (bounded) for its copies and instructions in
+// flight, frees its tensor memory and leaves without its output.  The weight
+// gradient (k_conv3d_wgrad_tc, below) runs on the same instructions with the
+// voxels as the reduction dimension.
 #include <cuda_bf16.h>
+
+#include <cmath>
 
 #include "kernels.h"
 #include "../../include/omega_b200_unet.h"
@@ -96,178 +109,363 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 
 }  // namespace tc
 
-template <int CIN, int COUT, bool RELU, bool MASK>
-__global__ void __launch_bounds__(128) k_conv3d_tc(const __nv_bfloat16 *__restrict__ in,
+// Shape of one convolution launch (conv_plan).
+struct ConvPlan {
+    int X, Y, Z, B;
+    int TX, TY, TZ;      // output voxels of a CTA's block
+    int P, S, T;         // staged line length, positions between M tiles, M tiles per plane
+    int ntx, nty, ntz;   // blocks per axis
+    int tiles;           // blocks in all
+    int ring;            // stages
+    int plane, stage;    // bytes of one 8-channel half plane (128-byte aligned) and of a stage
+    int cols;            // tensor-memory columns to allocate
+    int smem;            // dynamic shared memory
+};
+
+namespace tc {
+
+__device__ __forceinline__ uint64_t desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)((lbo >> 4) & 0x3FFF) << 16 |
+           (uint64_t)((sbo >> 4) & 0x3FFF) << 32 | (uint64_t)1 << 46;
+}
+
+}  // namespace tc
+
+// CO: output channels of a CTA; blockIdx.y picks which of COUT.
+template <int CIN, int COUT, int CO, bool RELU, bool MASK>
+__global__ void __launch_bounds__(256) k_conv3d_tc(const __grid_constant__ ConvPlan pl,
+                                                   const __nv_bfloat16 *__restrict__ in,
                                                    const __nv_bfloat16 *__restrict__ w,
                                                    const float *__restrict__ bias, __nv_bfloat16 *__restrict__ out,
-                                                   const __nv_bfloat16 *__restrict__ mask, int X, int Y, int Z,
-                                                   int64_t nvox) {
-    static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 128, "channel counts");
-    constexpr int TMEM_COLS = COUT <= 32 ? 32 : (COUT <= 64 ? 64 : 128);
-    constexpr int A_BYTES = tc::kM * 32, B_BYTES = COUT * 32;
-    constexpr int KSTEPS = 27 * (CIN / 16);
-    __shared__ __align__(1024) uint8_t sA[2][A_BYTES];
-    __shared__ __align__(1024) uint8_t sB[2][B_BYTES];
-    __shared__ __align__(8) uint64_t bars[2];
+                                                   const __nv_bfloat16 *__restrict__ mask) {
+    static_assert(CIN % 16 == 0 && COUT % CO == 0 && CO % 16 == 0 && CO <= 80, "channel counts");
+    constexpr int NCH = CIN / 16;             // 16-channel chunks: stages per input plane
+    constexpr int WBLOCK = 3 * CO * 32;       // weights of one (chunk, dy, dx): 3 dz taps x CO rows x 16 channels
+    constexpr int WBYTES = NCH * 9 * WBLOCK;
+    constexpr int kLoaders = 96;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(8) uint64_t full[4], empty[4], done, drained;
     __shared__ uint32_t tmem_base;
+    __shared__ int failed;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int co0 = blockIdx.y * CO;
     if (tid == 0) {
-        tc::mbar_init(tc::smem_u32(&bars[0]), 1);
-        tc::mbar_init(tc::smem_u32(&bars[1]), 1);
+        for (int i = 0; i < 4; ++i) {
+            tc::mbar_init(tc::smem_u32(&full[i]), kLoaders / 32);
+            tc::mbar_init(tc::smem_u32(&empty[i]), 1);
+        }
+        tc::mbar_init(tc::smem_u32(&done), 1);
+        tc::mbar_init(tc::smem_u32(&drained), 128);
+        failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc::smem_u32(&tmem_base)),
-                     "r"(TMEM_COLS)
+                     "r"(pl.cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
+    // weights: block (chunk, dy, dx), K half, row = (dz = +1, 0, -1) x CO, 8 channels
+    for (int i = tid; i < WBYTES / 16; i += 256) {
+        const int row = i % (3 * CO), q = i / (3 * CO);
+        const int h = q & 1, blk = q >> 1;
+        const int t9 = blk % 9, c = blk / 9;
+        const int tap = (2 - row / CO) * 9 + t9;
+        *reinterpret_cast<uint4 *>(smem + (size_t)i * 16) = __ldg(reinterpret_cast<const uint4 *>(
+            w + ((int64_t)tap * COUT + co0 + row % CO) * CIN + c * 16 + h * 8));
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = tmem_base;
+    const uint32_t wbase = tc::smem_u32(smem), ring = wbase + WBYTES;
+    const int nst = (pl.TZ + 2) * NCH;   // stages per block
+    const int mine = (int)blockIdx.x < pl.tiles ? (pl.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int total = mine * nst;
 
-    // this thread's A row: voxel v (its neighbours change per tap)
-    const int64_t v = (int64_t)blockIdx.x * tc::kM + tid;
-    const bool vin = v < nvox;
-    int x = 0, y = 0, z = 0;
-    int64_t b = 0;
-    if (vin) {
-        int64_t q = v;
-        x = (int)(q % X);
-        q /= X;
-        y = (int)(q % Y);
-        q /= Y;
-        z = (int)(q % Z);
-        b = q / Z;
-    }
-    const uint32_t idesc = tc::instr_desc(COUT);
-    // Step ks uses stage ks & 1; it is that stage's (ks >> 1)-th use, so the
-    // commit it waits for before refilling (step ks - 2) completed phase
-    // ((ks >> 1) - 1) & 1 of the stage's mbarrier.
-    int issued = 0;
-    bool ok = true;
-    for (int ks = 0; ks < KSTEPS; ++ks) {
-        const int tap = ks / (CIN / 16), c = (ks % (CIN / 16)) * 16;
-        const int s = ks & 1;
-        if (ks >= 2) {
-            if (!tc::mbar_wait(tc::smem_u32(&bars[s]), (uint32_t)((ks >> 1) - 1) & 1u)) ok = false;
-        }
-        if (!__syncthreads_and(ok)) {
-            ok = false;
-            break;
-        }
-        // A row of this thread: 16 channels of the tap-shifted voxel
-        {
-            const int xs = x + tap % 3 - 1, ys = y + (tap / 3) % 3 - 1, zs = z + tap / 9 - 1;
-            uint4 lo = make_uint4(0, 0, 0, 0), hi = lo;
-            if (vin && xs >= 0 && xs < X && ys >= 0 && ys < Y && zs >= 0 && zs < Z) {
-                const uint4 *p = reinterpret_cast<const uint4 *>(in + (((b * Z + zs) * Y + ys) * X + xs) * CIN + c);
-                lo = __ldg(p);
-                hi = __ldg(p + 1);
+    auto block_origin = [&](int k, int &x0, int &y0, int &z0, int &b) {
+        int tile = (int)blockIdx.x + k * (int)gridDim.x;
+        x0 = tile % pl.ntx * pl.TX;
+        tile /= pl.ntx;
+        y0 = tile % pl.nty * pl.TY;
+        tile /= pl.nty;
+        z0 = tile % pl.ntz * pl.TZ;
+        b = tile / pl.ntz;
+    };
+    auto fail = [&] {
+        atomicExch(&g_unet_error, 1);
+        *(volatile int *)&failed = 1;
+    };
+
+    if (warp >= 1 && warp <= 3) {
+        // loaders: stage it + lag is requested before stage `it` is handed over
+        const int j = tid - 32;
+        const int lag = pl.ring > 2 ? 2 : 1;
+        const int items = 2 * pl.P * (pl.TY + 2);
+        const uint32_t bar0 = tc::smem_u32(&full[0]);
+        auto hand_over = [&](int it) {
+            // (cp.async writes through the generic proxy, the tensor core reads through the async one)
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar0 + 8u * (it % pl.ring)) : "memory");
+        };
+        int x0 = 0, y0 = 0, z0 = 0, b = 0, it = 0;
+        bool ok = true;
+        for (int k = 0; k < mine && ok; ++k) {
+            block_origin(k, x0, y0, z0, b);
+            for (int st = 0; st < nst; ++st, ++it) {
+                const int slot = it % pl.ring, use = it / pl.ring;
+                if (use > 0) ok = tc::mbar_wait(tc::smem_u32(&empty[slot]), (uint32_t)(use - 1) & 1u);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    break;
+                }
+                const int zi = st / NCH, c = st - zi * NCH, z = z0 + zi - 1;
+                const bool zin = z >= 0 && z < pl.Z;
+                const uint32_t dst0 = ring + slot * pl.stage;
+                const __nv_bfloat16 *plane = in + ((int64_t)b * pl.Z + (zin ? z : 0)) * pl.Y * pl.X * CIN + c * 16;
+                // item i: half i & 1 of position i >> 1
+                int line = 0, x = j >> 1;
+                const int h = j & 1;
+                for (int i = j; i < items; i += kLoaders, x += kLoaders / 2) {
+                    while (x >= pl.P) {
+                        x -= pl.P;
+                        ++line;
+                    }
+                    const int gx = x0 + x - 1, gy = y0 + line - 1;
+                    const bool inside = zin && gx >= 0 && gx < pl.X && gy >= 0 && gy < pl.Y;
+                    const __nv_bfloat16 *src = inside ? plane + ((int64_t)gy * pl.X + gx) * CIN + h * 8 : in;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst0 + h * pl.plane + (i >> 1) * 16),
+                                 "l"(src), "r"(inside ? 16 : 0)
+                                 : "memory");
+                }
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+                if (it >= lag) {
+                    if (lag == 2)
+                        asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+                    else
+                        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+                    hand_over(it - lag);
+                }
             }
-            uint8_t *dst = sA[s] + (tid >> 3) * tc::kCoreGroup + (tid & 7) * 16;
-            *reinterpret_cast<uint4 *>(dst) = lo;
-            *reinterpret_cast<uint4 *>(dst + tc::kKHalf) = hi;
         }
-        // B rows: output channel co = tid, 16 input channels
-        if (tid < COUT) {
-            const uint4 *p = reinterpret_cast<const uint4 *>(w + ((int64_t)tap * COUT + tid) * CIN + c);
-            uint8_t *dst = sB[s] + (tid >> 3) * tc::kCoreGroup + (tid & 7) * 16;
-            *reinterpret_cast<uint4 *>(dst) = __ldg(p);
-            *reinterpret_cast<uint4 *>(dst + tc::kKHalf) = __ldg(p + 1);
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        if (ok)
+            for (int i = total > lag ? total - lag : 0; i < total; ++i) hand_over(i);
+        else if (lane == 0)
+            fail();
+    } else if (tid == 0) {
+        int it = 0;
+        bool ok = true;
+        for (int k = 0; k < mine && ok; ++k) {
+            // the previous block's sums have been read
+            if (k > 0) ok = tc::mbar_wait(tc::smem_u32(&drained), (uint32_t)(k - 1) & 1u);
+            for (int st = 0; st < nst && ok; ++st, ++it) {
+                const int slot = it % pl.ring;
+                ok = tc::mbar_wait(tc::smem_u32(&full[slot]), (uint32_t)(it / pl.ring) & 1u);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const int zr = st / NCH, c = st - zr * NCH;               // input plane z0 + zr - 1
+                const int lo = max(zr - 2, 0), hi = min(zr, pl.TZ - 1);   // output planes it adds to
+                const bool opens = c == 0 && zr < pl.TZ;                  // the last of them gets its first sum
+                const uint32_t a0 = ring + slot * pl.stage;
+                for (int t9 = 0; t9 < 9; ++t9) {
+                    const uint32_t a = a0 + (uint32_t)((t9 / 3) * pl.P + t9 % 3) * 16u;
+                    const uint32_t bw = wbase + (uint32_t)(c * 9 + t9) * WBLOCK;
+                    const uint32_t b = bw + (uint32_t)((lo - (zr - 2)) * CO) * 16u;
+                    const bool first = opens && t9 == 0;
+                    const int n = (hi - lo + 1 - (first ? 1 : 0)) * CO;
+                    for (int t = 0; t < pl.T; ++t) {
+                        const uint64_t da = tc::desc(a + (uint32_t)(t * pl.S) * 16u, pl.plane, 128);
+                        const uint32_t d = tmem + (uint32_t)((t * pl.TZ + lo) * CO);
+                        if (n > 0) tc::mma_issue(d, da, tc::desc(b, 3 * CO * 16, 128), tc::instr_desc(n), 1u);
+                        if (first)
+                            tc::mma_issue(tmem + (uint32_t)((t * pl.TZ + hi) * CO), da,
+                                          tc::desc(bw + 2 * CO * 16, 3 * CO * 16, 128), tc::instr_desc(CO), 0u);
+                    }
+                }
+                tc::mma_commit(tc::smem_u32(&empty[slot]));
+            }
+            // (on failure too: whoever waits for it is let go once the instructions in flight have ended)
+            if (!ok) fail();
+            tc::mma_commit(tc::smem_u32(&done));
         }
-        // make the generic-proxy smem writes visible to the tensor core
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+    } else if (warp >= 4) {
+        const int quarter = warp & 3;   // the tensor-memory lanes this warp can read
+        for (int k = 0; k < mine; ++k) {
+            const bool ok = tc::mbar_wait(tc::smem_u32(&done), (uint32_t)k & 1u) && !*(volatile int *)&failed;
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0) fail();
+                break;
+            }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            tc::mma_issue(tmem, tc::smem_desc(tc::smem_u32(sA[s])), tc::smem_desc(tc::smem_u32(sB[s])), idesc,
-                          ks > 0 ? 1u : 0u);
-            tc::mma_commit(tc::smem_u32(&bars[s]));
-        }
-        issued = ks + 1;
-    }
-    // the last commit tracks every MMA issued before it
-    if (ok) {
-        const int last = KSTEPS - 1;
-        if (!tc::mbar_wait(tc::smem_u32(&bars[last & 1]), (uint32_t)(last >> 1) & 1u)) ok = false;
-    }
-    if (!ok) {
-        // a commit never arrived: report, give the tensor core a bounded time
-        // to finish what it was given, and leave without the epilogue
-        if (tid == 0) atomicExch(&g_unet_error, 1);
-        if (issued > 0) tc::mbar_wait(tc::smem_u32(&bars[(issued - 1) & 1]), (uint32_t)((issued - 1) >> 1) & 1u);
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (ok) {
-        const int64_t vo = (int64_t)blockIdx.x * tc::kM + warp * 32 + lane;
+            int x0, y0, z0, b;
+            block_origin(k, x0, y0, z0, b);
+            for (int t = 0; t < pl.T; ++t) {
+                const int pos = t * pl.S + quarter * 32 + lane;
+                const int line = pos / pl.P, x = x0 + pos - line * pl.P, y = y0 + line;
+                const bool inside = pos - line * pl.P < pl.TX && line < pl.TY && x < pl.X && y < pl.Y;
+                for (int zo = 0; zo < pl.TZ && z0 + zo < pl.Z; ++zo) {
+                    const int64_t vo = (((int64_t)b * pl.Z + z0 + zo) * pl.Y + y) * pl.X + x;
 #pragma unroll
-        for (int c0 = 0; c0 < COUT; c0 += 16) {
-            float acc[16];
-            tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, acc);
-            if (vo < nvox) {
-                __nv_bfloat16 m16[16];
-                if (MASK) {
-                    const uint4 *mp = reinterpret_cast<const uint4 *>(mask + vo * COUT + c0);
-                    *reinterpret_cast<uint4 *>(m16) = __ldg(mp);
-                    *reinterpret_cast<uint4 *>(m16 + 8) = __ldg(mp + 1);
-                }
-                uint32_t packed[8];
+                    for (int c0 = 0; c0 < CO; c0 += 16) {
+                        float acc[16];
+                        __syncwarp();
+                        tc::tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((t * pl.TZ + zo) * CO + c0), acc);
+                        if (inside) {
+                            __nv_bfloat16 m16[16];
+                            if (MASK) {
+                                const uint4 *mp = reinterpret_cast<const uint4 *>(mask + vo * COUT + co0 + c0);
+                                *reinterpret_cast<uint4 *>(m16) = __ldg(mp);
+                                *reinterpret_cast<uint4 *>(m16 + 8) = __ldg(mp + 1);
+                            }
+                            uint32_t packed[8];
 #pragma unroll
-                for (int i = 0; i < 16; i += 2) {
-                    float lo = acc[i], hi = acc[i + 1];
-                    if (bias) {
-                        lo += __ldg(bias + c0 + i);
-                        hi += __ldg(bias + c0 + i + 1);
+                            for (int i = 0; i < 16; i += 2) {
+                                float lo = acc[i], hi = acc[i + 1];
+                                if (bias) {
+                                    lo += __ldg(bias + co0 + c0 + i);
+                                    hi += __ldg(bias + co0 + c0 + i + 1);
+                                }
+                                if (RELU) {
+                                    lo = fmaxf(lo, 0.f);
+                                    hi = fmaxf(hi, 0.f);
+                                }
+                                if (MASK) {
+                                    if (!(__bfloat162float(m16[i]) > 0.f)) lo = 0.f;
+                                    if (!(__bfloat162float(m16[i + 1]) > 0.f)) hi = 0.f;
+                                }
+                                const __nv_bfloat162 pr = __floats2bfloat162_rn(lo, hi);
+                                packed[i / 2] = *reinterpret_cast<const uint32_t *>(&pr);
+                            }
+                            uint4 *op = reinterpret_cast<uint4 *>(out + vo * COUT + co0 + c0);
+                            op[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                            op[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                        }
                     }
-                    if (RELU) {
-                        lo = fmaxf(lo, 0.f);
-                        hi = fmaxf(hi, 0.f);
-                    }
-                    if (MASK) {
-                        if (!(__bfloat162float(m16[i]) > 0.f)) lo = 0.f;
-                        if (!(__bfloat162float(m16[i + 1]) > 0.f)) hi = 0.f;
-                    }
-                    const __nv_bfloat162 pr = __floats2bfloat162_rn(lo, hi);
-                    packed[i / 2] = *reinterpret_cast<const uint32_t *>(&pr);
                 }
-                uint4 *op = reinterpret_cast<uint4 *>(out + vo * COUT + c0);
-                op[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                op[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
             }
+            // the next block's instructions overwrite the accumulators
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&drained)) : "memory");
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(pl.cols) : "memory");
+    }
 }
 
 #define OMB_TC_SHAPES(X) X(16, 16) X(16, 32) X(32, 32) X(32, 64) X(64, 64) X(96, 32) X(48, 16) \
     X(32, 16) X(64, 32) X(32, 96) X(16, 48)
 
+// Dynamic shared memory of a CTA that leaves room for a second one (228 KB per
+// SM, 1 KB of it per CTA reserved and 1 KB static).
+constexpr int kHalfSmem = 111 * 1024;
+
+// Block shape of a convolution: the least estimated time per output voxel over
+// the blocks that fit.  An instruction takes 32 clocks for its 4 KB of A plus
+// one per 4 columns; a staged 16-byte row costs the loaders about a third; two
+// CTAs on an SM (half the shared memory and tensor-memory columns each) hide
+// the epilogue, and a last wave that is partly empty counts in full.
+static ConvPlan conv_plan(int cin, int co, int groups, int X, int Y, int Z, int B) {
+    ConvPlan best{};
+    double best_cost = 1e300;
+    const int nch = cin / 16, wbytes = nch * 9 * 3 * co * 32;
+    for (int occ = 2; occ >= 1; --occ) {
+        const int max_cols = occ == 2 ? 256 : 512, max_smem = occ == 2 ? kHalfSmem : 226 * 1024;
+        for (int ty = 1; ty <= 32 && (ty <= Y || ty == 1); ++ty)
+            for (int tz = 1; tz <= 8 && (tz <= Z || tz == 1); ++tz) {
+                ConvPlan p{X, Y, Z, B};
+                p.ntx = (X + 127) / 128;
+                p.TX = (X + p.ntx - 1) / p.ntx;
+                p.TY = ty;
+                p.TZ = tz;
+                p.P = p.TX + 2;
+                p.S = p.TX == 128 ? p.P : 128;
+                p.T = p.TX == 128 ? ty : ((ty - 1) * p.P + p.TX + 127) / 128;
+                if (p.T * tz * co > max_cols) continue;
+                for (p.cols = 32; p.cols < p.T * tz * co;) p.cols *= 2;
+                p.plane = ((ty + 2) * p.P * 16 + 127) / 128 * 128;
+                p.stage = 2 * p.plane;
+                // rows past the plane are read by the last M tile and dropped
+                const int over = ((p.T - 1) * p.S + 128 + 2 * p.P + 2) * 16;
+                const int pad = over > p.plane ? over - p.plane : 0;
+                p.ring = 4;
+                while (p.ring > 1 && wbytes + p.ring * p.stage + pad > max_smem) --p.ring;
+                if (p.ring < 2) continue;
+                p.smem = wbytes + p.ring * p.stage + pad;
+                p.nty = (Y + ty - 1) / ty;
+                p.ntz = (Z + tz - 1) / tz;
+                const int64_t tiles = (int64_t)p.ntx * p.nty * p.ntz * B;
+                if (tiles > 0x7fffffff / (10 * nch)) continue;   // (stage counters are 32-bit)
+                p.tiles = (int)tiles;
+                const double mma = (double)(tz + 2) * nch * 9 * p.T * (32 + co * 0.75 * tz / (tz + 2));
+                const double load = 0.35 * (tz + 2) * nch * 2 * (ty + 2) * p.P;
+                const double epi = 60.0 * p.T * tz * co / 16;
+                const double busy = (mma > load ? mma : load) * (p.ring > 2 ? 1.0 : 1.2);
+                const double per = occ == 2 ? (busy > epi ? busy : epi) : busy + epi;
+                const double slots = (double)num_sms() * occ;
+                const double cost = ceil(tiles * (double)groups / slots) * slots * per / occ;
+                if (cost < best_cost * (occ == 2 ? 1.0 : 0.999)) {
+                    best_cost = cost;
+                    best = p;
+                }
+            }
+    }
+    return best;
+}
+
+template <int CIN, int COUT, int CO, bool RELU, bool MASK>
+static int conv_launch(const ConvPlan &pl, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias,
+                       __nv_bfloat16 *out, const __nv_bfloat16 *mask, cudaStream_t st) {
+    auto kernel = k_conv3d_tc<CIN, COUT, CO, RELU, MASK>;
+    OMB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem));
+    const int occ = pl.smem <= kHalfSmem && pl.cols <= 256 ? 2 : 1;
+    const int slots = num_sms() * occ / (COUT / CO);
+    const int grid = pl.tiles < slots ? pl.tiles : slots;
+    kernel<<<dim3(grid, COUT / CO), 256, pl.smem, st>>>(pl, in, w, bias, out, mask);
+    OMB_LAUNCH_CHECK("tcgen05 conv launch");
+    return OMB_OK;
+}
+
+template <int CIN, int COUT>
+static int conv_shape(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias, __nv_bfloat16 *out,
+                      const __nv_bfloat16 *mask, int relu, int X, int Y, int Z, int B, cudaStream_t st) {
+    // output channels of a CTA: all of them up to 48 (their weights and three
+    // planes of accumulators must fit), else thirds or halves
+    constexpr int CO = COUT <= 48 ? COUT : (COUT % 48 == 0 ? 48 : 32);
+    // the plans of the last sizes this thread used (the search takes some
+    // microseconds; a plan depends on the sizes alone)
+    static thread_local ConvPlan plans[8];
+    static thread_local int next = 0;
+    const ConvPlan *found = nullptr;
+    for (const ConvPlan &p : plans)
+        if (p.tiles > 0 && p.X == X && p.Y == Y && p.Z == Z && p.B == B) found = &p;
+    if (!found) {
+        plans[next] = conv_plan(CIN, CO, COUT / CO, X, Y, Z, B);
+        found = &plans[next];
+        next = (next + 1) % 8;
+    }
+    const ConvPlan pl = *found;
+    if (pl.tiles == 0) return set_error(OMB_ERR_UNSUPPORTED, "conv volume too large");
+    if (mask) return conv_launch<CIN, COUT, CO, false, true>(pl, in, w, bias, out, mask, st);
+    if (relu) return conv_launch<CIN, COUT, CO, true, false>(pl, in, w, bias, out, mask, st);
+    return conv_launch<CIN, COUT, CO, false, false>(pl, in, w, bias, out, mask, st);
+}
+
 int unet_conv_tc(int cin, int cout, const void *in, const void *w, const float *bias, void *out, const void *mask,
                  int relu, int X, int Y, int Z, int B, cudaStream_t st) {
     if (X <= 0 || Y <= 0 || Z <= 0 || B <= 0) return set_error(OMB_ERR_INVALID, "bad conv volume");
-    const int64_t nvox = (int64_t)X * Y * Z * B;
-    const int64_t blocks = (nvox + tc::kM - 1) / tc::kM;
-    if (blocks > 2147483647) return set_error(OMB_ERR_UNSUPPORTED, "conv volume too large");
     const auto *i = static_cast<const __nv_bfloat16 *>(in), *wt = static_cast<const __nv_bfloat16 *>(w),
                *mk = static_cast<const __nv_bfloat16 *>(mask);
     auto *o = static_cast<__nv_bfloat16 *>(out);
-    const unsigned grid = (unsigned)blocks;
-#define X(ci, co)                                                                                   \
-    if (cin == ci && cout == co) {                                                                  \
-        if (mask)                                                                                   \
-            k_conv3d_tc<ci, co, false, true><<<grid, 128, 0, st>>>(i, wt, bias, o, mk, X, Y, Z, nvox);  \
-        else if (relu)                                                                              \
-            k_conv3d_tc<ci, co, true, false><<<grid, 128, 0, st>>>(i, wt, bias, o, mk, X, Y, Z, nvox);  \
-        else                                                                                        \
-            k_conv3d_tc<ci, co, false, false><<<grid, 128, 0, st>>>(i, wt, bias, o, mk, X, Y, Z, nvox); \
-        OMB_LAUNCH_CHECK("tcgen05 conv launch");                                                    \
-        return OMB_OK;                                                                              \
-    }
+#define X(ci, co) \
+    if (cin == ci && cout == co) return conv_shape<ci, co>(i, wt, bias, o, mk, relu, X, Y, Z, B, st);
     OMB_TC_SHAPES(X)
 #undef X
     return set_error(OMB_ERR_UNSUPPORTED, "conv shape " + std::to_string(cin) + "->" + std::to_string(cout) +
