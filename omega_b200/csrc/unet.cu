@@ -13,8 +13,9 @@
 //            W'[tap][ci][co] = W[26 - tap][co][ci] (off(26 - tap) = -off(tap)),
 //            with the next ReLU's derivative fused as a mask on the output
 //   wgrad    dW[tap][co][ci] = sum_v dz[v][co] in[v+off(tap)][ci]: voxels are
-//            the GEMM's K; tiles of 128 voxels staged in shared memory and read
-//            transposed with ldmatrix.trans, partial sums added with FP32 atomics.
+//            the GEMM's K; lines of voxels with their halo staged once in shared
+//            memory and read transposed and shifted with ldmatrix.trans, partial
+//            sums added with FP32 atomics.
 #include <cuda_bf16.h>
 
 #include "kernels.h"
@@ -112,101 +113,184 @@ __global__ void __launch_bounds__(128) k_conv3d(const bf16 *__restrict__ in, con
 }
 
 // ---------------------------------------------------------------------------
-// Weight gradient.  grid = (chunks, 27); block = 4 warps; each block reduces
-// `per_block` voxels (multiple of 128) for one tap.
+// Weight gradient.  A stage is TY lines of dz with a one-voxel halo in x and
+// TY + 2 lines of the input plane dz away (blockIdx.y picks dz = -1, 0, 1),
+// both as planes of 8 channels with 16-byte rows in voxel order, copied with
+// cp.async into a ring of stages; ldmatrix reads any 8 consecutive voxels
+// without bank conflicts.  A shift by dx is put on the dz operand and a shift
+// by dy on the input, so the 9 taps of a stage need 3 + 3 operand loads per 16
+// voxels.  A warp holds the three dx taps of one dy for MTW x NTW tiles of 16
+// output x 8 input channels (up to 96 accumulators); MS x NS warps cover the
+// channels and KS of them share the voxels.  Bound by the tensor cores'
+// m16n8k16 rate with the operand loads beside it; one tap per block of a 27-fold
+// grid, as it was before, staged both operands again for each tap
+// (training step at 128 x 128 x 64 x 4: 19.1 -> 11.8 ms).
 // ---------------------------------------------------------------------------
+struct WgradPlan {
+    int X, Y, Z, B;
+    int TX, TY;            // voxels of a stage (TX a multiple of 16; past the line's end the input is zero)
+    int ntx, nty, tiles;   // stages in all
+    int ring;              // stages in shared memory
+    int in_plane, dz_plane, dz_off, stage;   // bytes
+    int flush;             // stages whose sums a warp adds up before they go to dw
+    int smem;
+};
+
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_conv3d_wgrad(const bf16 *__restrict__ in, const bf16 *__restrict__ dz,
-                                                      float *__restrict__ dw, int X, int Y, int Z, int64_t nvox,
-                                                      int per_block) {
-    constexpr int SA = COUT + 8, SB = CIN + 8;  // padded smem rows (bank spread for ldmatrix)
-    __shared__ __align__(16) bf16 sA[128 * SA];
-    __shared__ __align__(16) bf16 sB[128 * SB];
-    constexpr int MT = COUT / 16, NT = CIN / 8, TILES = MT * NT;
-    constexpr int PER_WARP = (TILES + 3) / 4;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tap = blockIdx.y;
-    const int ddz = tap / 9 - 1, ddy = (tap / 3) % 3 - 1, ddx = tap % 3 - 1;
-    float acc[PER_WARP][4];
+struct WgradShape {
+    static constexpr int MT = COUT / 16, NT = CIN / 8;
+    static constexpr int MTW = MT <= 3 ? MT : 2, NTW = NT <= 2 ? NT : (MTW == 1 && NT == 6 ? 6 : (MTW == 3 ? 2 : 4));
+    static constexpr int MS = MT / MTW, NS = NT / NTW;
+    static constexpr int KS = MS * NS >= 4 ? 1 : 4 / (MS * NS);
+    static constexpr int kWarps = 3 * MS * NS * KS, kThreads = 32 * kWarps;
+    static_assert(MT % MTW == 0 && NT % NTW == 0 && NTW % 2 == 0 && 3 * MTW * NTW * 4 <= 96, "wgrad tiles");
+    static_assert(kThreads % (CIN / 8) == 0 && kThreads % (COUT / 8) == 0, "copy loops");
+};
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(WgradShape<CIN, COUT>::kThreads, 1)
+    k_conv3d_wgrad(const __grid_constant__ WgradPlan pl, const bf16 *__restrict__ in, const bf16 *__restrict__ dz,
+                   float *__restrict__ dw) {
+    using S = WgradShape<CIN, COUT>;
+    constexpr int MTW = S::MTW, NTW = S::NTW, CI8 = CIN / 8, CO8 = COUT / 8;
+    extern __shared__ __align__(128) uint8_t wsmem[];
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(wsmem);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int dy = warp % 3, part = warp / 3;
+    const int ks = part % S::KS, ns = part / S::KS % S::NS, ms = part / S::KS / S::NS;
+    const int dzi = (int)blockIdx.y - 1;
+    const int P = pl.TX + 2;
+    float acc[3][MTW][NTW][4];
+    auto clear = [&] {
 #pragma unroll
-    for (int i = 0; i < PER_WARP; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-    const int64_t v_begin = (int64_t)blockIdx.x * per_block;
-    const int64_t v_end = min(v_begin + (int64_t)per_block, nvox);
-    for (int64_t v0 = v_begin; v0 < v_end; v0 += 128) {
-        // stage: thread r loads voxel v0 + r's dz row and its tap-shifted input row
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int m = 0; m < MTW; ++m)
+#pragma unroll
+                for (int n = 0; n < NTW; ++n) acc[d][m][n][0] = acc[d][m][n][1] = acc[d][m][n][2] = acc[d][m][n][3] = 0.f;
+    };
+    clear();
+    const int mine = (int)blockIdx.x < pl.tiles ? (pl.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    auto copy16 = [](uint32_t dst, const bf16 *src, bool ok) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+    };
+    // requests stage k of this block's sequence
+    auto load = [&](int k) {
+        int tile = (int)blockIdx.x + k * (int)gridDim.x;
+        const int x0 = tile % pl.ntx * pl.TX;
+        tile /= pl.ntx;
+        const int y0 = tile % pl.nty * pl.TY;
+        tile /= pl.nty;
+        const int z = tile % pl.Z, b = tile / pl.Z, zi = z + dzi;
+        const uint32_t st = base + (uint32_t)(k % pl.ring) * pl.stage;
+        const bool zin = zi >= 0 && zi < pl.Z;
+        const bf16 *ip = in + ((int64_t)b * pl.Z + (zin ? zi : 0)) * pl.Y * pl.X * CIN;
+        const bf16 *dp = dz + ((int64_t)b * pl.Z + z) * pl.Y * pl.X * COUT;
         {
-            const int r = threadIdx.x;
-            const int64_t v = v0 + r;
-            bool ok = v < v_end;
-            int64_t src = 0;
-            if (ok) {
-                const int x = (int)(v % X);
-                const int64_t q = v / X;
-                const int yv = (int)(q % Y);
-                const int64_t q2 = q / Y;
-                const int zv = (int)(q2 % Z);
-                const int64_t bb = q2 / Z;
-                const int xs = x + ddx, ys = yv + ddy, zs = zv + ddz;
-                if (xs >= 0 && xs < X && ys >= 0 && ys < Y && zs >= 0 && zs < Z)
-                    src = ((bb * Z + zs) * Y + ys) * X + xs;
-                else
-                    src = -1;
-            }
-            const uint4 zero4 = make_uint4(0, 0, 0, 0);
-#pragma unroll
-            for (int c = 0; c < COUT; c += 8)
-                *reinterpret_cast<uint4 *>(sA + r * SA + c) =
-                    ok ? __ldg(reinterpret_cast<const uint4 *>(dz + v * COUT + c)) : zero4;
-#pragma unroll
-            for (int c = 0; c < CIN; c += 8)
-                *reinterpret_cast<uint4 *>(sB + r * SB + c) =
-                    (ok && src >= 0) ? __ldg(reinterpret_cast<const uint4 *>(in + src * CIN + c)) : zero4;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 128; k += 16) {
-#pragma unroll
-            for (int i = 0; i < PER_WARP; ++i) {
-                const int tile = warp + 4 * i;
-                if (tile < TILES) {
-                    const int mt = tile / NT, nt = tile % NT;
-                    // A = dz^T (co x voxel): ldmatrix.x4.trans of sA rows k.., columns mt*16..
-                    const int mi = lane >> 3, rr = lane & 7;
-                    const bf16 *pa = sA + (k + rr + (mi >> 1) * 8) * SA + mt * 16 + (mi & 1) * 8;
-                    uint32_t a0, a1, a2, a3;
-                    const uint32_t sa = (uint32_t)__cvta_generic_to_shared(pa);
-                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                                 : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
-                                 : "r"(sa));
-                    // B = input (voxel x ci): ldmatrix.x2.trans of sB rows k.., columns nt*8..
-                    const int mb = (lane >> 3) & 1;
-                    const bf16 *pb = sB + (k + rr + mb * 8) * SB + nt * 8;
-                    uint32_t b0, b1;
-                    const uint32_t sb = (uint32_t)__cvta_generic_to_shared(pb);
-                    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-                                 : "=r"(b0), "=r"(b1)
-                                 : "r"(sb));
-                    mma_bf16(acc[i], a0, a1, a2, a3, b0, b1);
+            const int c = tid % CI8;
+            int x = tid / CI8, line = 0;
+            const uint32_t dst = st + c * pl.in_plane;
+            for (int q = x; q < (pl.TY + 2) * pl.TX; q += S::kThreads / CI8, x += S::kThreads / CI8) {
+                while (x >= pl.TX) {
+                    x -= pl.TX;
+                    ++line;
                 }
+                const int gx = x0 + x, gy = y0 + line - 1;
+                const bool ok = zin && gx < pl.X && gy >= 0 && gy < pl.Y;
+                copy16(dst + q * 16, ok ? ip + ((int64_t)gy * pl.X + gx) * CIN + c * 8 : in, ok);
             }
         }
-        __syncthreads();
-    }
-    // D fragment: rows (co) mt*16 + g (+8), columns (ci) nt*8 + 2t (+1)
-    const int g = lane >> 2, t = lane & 3;
+        {
+            const int c = tid % CO8;
+            int x = tid / CO8, line = 0;
+            const uint32_t dst = st + pl.dz_off + c * pl.dz_plane;
+            for (int q = x; q < pl.TY * P; q += S::kThreads / CO8, x += S::kThreads / CO8) {
+                while (x >= P) {
+                    x -= P;
+                    ++line;
+                }
+                const int gx = x0 + x - 1, gy = y0 + line;
+                const bool ok = gx >= 0 && gx < pl.X && gy < pl.Y;
+                copy16(dst + q * 16, ok ? dp + ((int64_t)gy * pl.X + gx) * COUT + c * 8 : dz, ok);
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    auto flush = [&] {
+        const int g = lane >> 2, t = lane & 3;
 #pragma unroll
-    for (int i = 0; i < PER_WARP; ++i) {
-        const int tile = warp + 4 * i;
-        if (tile < TILES) {
-            const int mt = tile / NT, nt = tile % NT;
-            float *d = dw + (int64_t)tap * COUT * CIN;
-            const int co = mt * 16 + g, ci = nt * 8 + 2 * t;
-            atomicAdd(d + co * CIN + ci, acc[i][0]);
-            atomicAdd(d + co * CIN + ci + 1, acc[i][1]);
-            atomicAdd(d + (co + 8) * CIN + ci, acc[i][2]);
-            atomicAdd(d + (co + 8) * CIN + ci + 1, acc[i][3]);
+        for (int d = 0; d < 3; ++d) {
+            float *dt = dw + (int64_t)((dzi + 1) * 9 + dy * 3 + d) * COUT * CIN;
+#pragma unroll
+            for (int m = 0; m < MTW; ++m)
+#pragma unroll
+                for (int n = 0; n < NTW; ++n) {
+                    const int co = (ms * MTW + m) * 16 + g, ci = (ns * NTW + n) * 8 + 2 * t;
+                    atomicAdd(dt + co * CIN + ci, acc[d][m][n][0]);
+                    atomicAdd(dt + co * CIN + ci + 1, acc[d][m][n][1]);
+                    atomicAdd(dt + (co + 8) * CIN + ci, acc[d][m][n][2]);
+                    atomicAdd(dt + (co + 8) * CIN + ci + 1, acc[d][m][n][3]);
+                }
+        }
+    };
+    for (int k = 0; k < pl.ring - 1; ++k) {
+        if (k < mine)
+            load(k);
+        else
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+    }
+    // ldmatrix rows of this lane: matrix mi, row rr
+    const int mi = lane >> 3, rr = lane & 7;
+    const int steps = pl.TX / 16, total = steps * pl.TY;
+    for (int k = 0; k < mine; ++k) {
+        if (pl.ring == 3)
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        else
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();   // stage k is here for everybody, and everybody is done with stage k - 1
+        if (k + pl.ring - 1 < mine)
+            load(k + pl.ring - 1);
+        else
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const uint32_t st = base + (uint32_t)(k % pl.ring) * pl.stage;
+        // input: matrices (voxels 0-7 / 8-15) of two channel planes; dz: two planes for each half of the voxels
+        const uint32_t ib = st + (ns * NTW + (mi >> 1)) * pl.in_plane + ((mi & 1) * 8 + rr) * 16;
+        const uint32_t db = st + pl.dz_off + (ms * MTW * 2 + (mi & 1)) * pl.dz_plane + ((mi >> 1) * 8 + rr) * 16;
+        for (int s = ks; s < total; s += S::KS) {
+            const int line = s / steps, x = (s - line * steps) * 16;
+            const uint32_t ia = ib + (uint32_t)((line + dy) * pl.TX + x) * 16u;
+            const uint32_t da = db + (uint32_t)(line * P + x) * 16u;
+            uint32_t bq[NTW / 2][4];
+#pragma unroll
+            for (int n = 0; n < NTW / 2; ++n) ldmatrix_x4_trans(bq[n], ia + 2 * n * pl.in_plane);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                // tap dx = d - 1 pairs input voxel u with dz voxel u - dx, staged at u - dx + 1
+                uint32_t aq[MTW][4];
+#pragma unroll
+                for (int m = 0; m < MTW; ++m) ldmatrix_x4_trans(aq[m], da + (2 - d) * 16 + 2 * m * pl.dz_plane);
+#pragma unroll
+                for (int m = 0; m < MTW; ++m)
+#pragma unroll
+                    for (int n = 0; n < NTW; ++n)
+                        mma_bf16(acc[d][m][n], aq[m][0], aq[m][1], aq[m][2], aq[m][3], bq[n / 2][(n & 1) * 2],
+                                 bq[n / 2][(n & 1) * 2 + 1]);
+            }
+        }
+        // sums of at most about 8192 voxels are added up before they go to memory
+        if ((k + 1) % pl.flush == 0 && k + 1 < mine) {
+            flush();
+            clear();
         }
     }
+    if (mine > 0) flush();
 }
 
 // Bias gradient: db[co] = sum_v dz[v][co] (FP32 atomics per block).
@@ -505,20 +589,49 @@ int unet_conv(int cin, int cout, const void *in, const void *w, const float *bia
                                               " is not built");
 }
 
+// The largest stage (at most 8 lines: the input's two halo lines weigh less)
+// of which three, or else two, fit an SM's shared memory.
+template <int CIN, int COUT>
+static int launch_wgrad(const bf16 *in, const bf16 *dz, float *dw, int X, int Y, int Z, int B, cudaStream_t st) {
+    using S = WgradShape<CIN, COUT>;
+    WgradPlan p{X, Y, Z, B};
+    p.ntx = (X + 127) / 128;
+    p.TX = ((X + p.ntx - 1) / p.ntx + 15) / 16 * 16;
+    // planes start 16 to 64 bytes apart modulo 128, so that the copies of
+    // neighbouring channels of a voxel meet different banks
+    auto plane = [](int rows, int planes) { return (rows * 16 + 127) / 128 * 128 + (planes <= 2 ? 64 : (planes <= 4 ? 32 : 16)); };
+    for (p.ring = 3; p.ring >= 2 && !p.smem; --p.ring) {
+        for (p.TY = Y < 8 ? Y : 8; p.TY >= 1; --p.TY) {
+            p.in_plane = plane((p.TY + 2) * p.TX, CIN / 8);
+            p.dz_plane = plane(p.TY * (p.TX + 2), COUT / 8);
+            p.dz_off = (p.in_plane * (CIN / 8) + 127) / 128 * 128;
+            p.stage = (p.dz_off + p.dz_plane * (COUT / 8) + 127) / 128 * 128;
+            if (p.ring * p.stage <= 226 * 1024) {
+                p.smem = p.ring * p.stage;
+                break;
+            }
+        }
+        if (p.smem) break;
+    }
+    p.nty = (Y + p.TY - 1) / p.TY;
+    const int64_t tiles = (int64_t)p.ntx * p.nty * Z * B;
+    if (!p.smem || tiles > 2147483647) return set_error(OMB_ERR_UNSUPPORTED, "wgrad volume too large");
+    p.tiles = (int)tiles;
+    p.flush = 8192 * S::KS / (p.TX * p.TY) > 1 ? 8192 * S::KS / (p.TX * p.TY) : 1;
+    auto kernel = k_conv3d_wgrad<CIN, COUT>;
+    OMB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, p.smem));
+    const int blocks = num_sms() / 3 > 0 ? num_sms() / 3 : 1;
+    kernel<<<dim3(p.tiles < blocks ? p.tiles : blocks, 3), S::kThreads, p.smem, st>>>(p, in, dz, dw);
+    OMB_LAUNCH_CHECK("wgrad launch");
+    return OMB_OK;
+}
+
 int unet_conv_wgrad(int cin, int cout, const void *in, const void *dz, float *dw, int X, int Y, int Z, int B,
                     cudaStream_t st) {
-    const int64_t nvox = (int64_t)X * Y * Z * B;
-    const int per_block = 128 * 64;
-    const int64_t chunks = (nvox + per_block - 1) / per_block;
-    if (chunks > 2147483647) return set_error(OMB_ERR_UNSUPPORTED, "wgrad volume too large");
-    dim3 grid((unsigned)chunks, 27);
+    if ((int64_t)X * Y * Z * B <= 0) return OMB_OK;
     const bf16 *i = static_cast<const bf16 *>(in), *d = static_cast<const bf16 *>(dz);
-#define X(ci, co)                                                                                          \
-    if (cin == ci && cout == co) {                                                                         \
-        k_conv3d_wgrad<ci, co><<<grid, 128, 0, st>>>(i, d, dw, X, Y, Z, nvox, per_block);                  \
-        OMB_LAUNCH_CHECK("wgrad launch");                                                                  \
-        return OMB_OK;                                                                                     \
-    }
+#define X(ci, co) \
+    if (cin == ci && cout == co) return launch_wgrad<ci, co>(i, d, dw, X, Y, Z, B, st);
     OMB_CONV_SHAPES(X)
 #undef X
     return set_error(OMB_ERR_UNSUPPORTED, "wgrad shape is not built");
