@@ -61,3 +61,42 @@ def test_conv_and_wgrad_at_ragged_volumes(cuda, ci, co, X, Y, Z, B):
     flag = ctypes.c_int32(-1)
     _native.call("omb_unet_take_error", ctypes.byref(flag))
     assert flag.value == 0
+
+
+@pytest.mark.parametrize("c,offset", [(16, 0), (32, 0), (24, 0), (12, 0), (16, 1)])
+def test_resampling_kernels(cuda, c, offset):
+    """8 channels per thread (multiples of 8, aligned) and element by element
+    (12 channels; a tensor that starts 2 bytes off)."""
+    import torch
+    from omega_b200 import _native
+    X, Y, Z, B, cs = 6, 10, 4, 2, 16 if c % 8 == 0 else 4
+    g = torch.Generator(device=cuda).manual_seed(c)
+
+    def t(*shape):
+        n = int(np.prod(shape))
+        buf = torch.randn(n + offset, generator=g, device=cuda).bfloat16()
+        return buf[offset:].view(*shape)
+
+    full, half = t(B, Z, Y, X, c), t(B, Z // 2, Y // 2, X // 2, c)
+    out = t(B, Z // 2, Y // 2, X // 2, c)
+    _native.call("omb_unet_avgpool", P(full), P(out), X, Y, Z, B, c, 0, _st(cuda))
+    pool = full.float().view(B, Z // 2, 2, Y // 2, 2, X // 2, 2, c).mean((2, 4, 6))
+    assert torch.allclose(out.float(), pool, atol=1e-2, rtol=1e-2)
+    up = lambda v: v.repeat_interleave(2, 1).repeat_interleave(2, 2).repeat_interleave(2, 3)  # noqa: E731
+    din = full.clone() if offset == 0 else t(B, Z, Y, X, c)
+    want = din.float() + 0.125 * up(half.float())
+    _native.call("omb_unet_avgpool", P(half), P(din), X, Y, Z, B, c, 1, _st(cuda))
+    assert torch.allclose(din.float(), want, atol=2e-2, rtol=1e-2)
+    skip, cat = t(B, Z, Y, X, cs), t(B, Z, Y, X, c + cs)
+    _native.call("omb_unet_up_concat", P(half), P(skip), P(cat), X, Y, Z, B, c, cs, _st(cuda))
+    assert torch.equal(cat, torch.cat([up(half), skip], -1))
+    dlow, dskip = t(B, Z // 2, Y // 2, X // 2, c), t(B, Z, Y, X, cs)
+    want_skip = dskip.float() + cat[..., c:].float()
+    _native.call("omb_unet_up_concat_bwd", P(cat), P(dlow), P(dskip), X, Y, Z, B, c, cs, _st(cuda))
+    want_low = cat[..., :c].float().view(B, Z // 2, 2, Y // 2, 2, X // 2, 2, c).sum((2, 4, 6))
+    assert torch.allclose(dlow.float(), want_low, atol=5e-2, rtol=1e-2)
+    assert torch.allclose(dskip.float(), want_skip, atol=3e-2, rtol=1e-2)
+    d = t(B, Z, Y, X, c)
+    want = torch.where(full.float() > 0, d, torch.zeros_like(d))
+    _native.call("omb_unet_relu_mask", P(d), P(full), d.numel(), _st(cuda))
+    assert torch.equal(d, want)
