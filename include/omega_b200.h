@@ -263,7 +263,7 @@ typedef struct omb_tuning {
     uint32_t struct_size;            /* sizeof(omb_tuning) */
     int32_t siddon_blocks_per_sm;    /* 1..32 (default 8): grid of the grid-stride Siddon kernels */
     int32_t siddon_frames_per_walk;  /* 1, 2, 4, 8 (default 8): most frames sharing one ray walk */
-    int32_t bdd_fp_columns;          /* 8, 16 (default 8): type-5 forward, detector columns per thread */
+    int32_t bdd_fp_columns;          /* 8, 16 (default 16 where the staged kernel fills the GPU with it, else 8): type-5 forward, detector columns per thread */
     int32_t bdd_bp_zrun;             /* 4, 8, 16 (default 16 where the staged kernel fills the GPU with it, else 8): type-5 backward, voxels along z per thread */
     int32_t bdd_fp_block_rows;       /* 4, 8 (default 8): type-5 forward, warps per block */
     int32_t bdd_bp_block_rows;       /* 4, 8 (default 8): type-5 backward, warps per block */

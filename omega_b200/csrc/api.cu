@@ -523,10 +523,18 @@ int omb_create(const omb_geometry_desc *desc, omb_handle **out) {
     g.my = desc->by + (float)desc->ny * desc->dy;
     g.mz = desc->bz + (float)desc->nz * desc->dz;
     h->n_img = (int64_t)desc->nx * desc->ny * desc->nz;
-    // Staged type-5 backprojection (bdd_bp_tma_supported): runs of 16 voxels
-    // share a footprint and a view's set-up among twice as many as 8 (90 views
-    // of 512 x 512, 256^3: 3.61 -> 2.94 ms) where the CTAs (32 x 4 columns of
-    // voxels) still fill every SM.
+    // Staged type-5 kernels (bdd_fp_tma_supported, bdd_bp_tma_supported): 16
+    // detector columns per thread share a slice's set-up among twice as many as
+    // 8 (90 views of 512 x 512, 256^3: 3.42 -> 2.75 ms, with the other changes
+    // of that kernel), and runs of 16 voxels a footprint and a view's set-up
+    // (back 3.61 -> 2.94 ms) -- where their CTAs (32 x 64 pixels of a view; 32 x 4
+    // columns of voxels) still fill every SM.  The unstaged kernels spend their
+    // time in memory accesses and lose with the wider threads (133 x 133 x 80,
+    // 161 x 79 x 80 views: forward, dual and back 1.78 against 2.17 ms).
+    if (desc->fp_type == 5 && desc->nx % 4 == 0 && desc->ny % 4 == 0 && desc->n_cols_d >= 64 &&
+        (int64_t)((desc->n_rows_d + 31) / 32) * ((desc->n_cols_d + 63) / 64) * (desc->n_proj / desc->n_subsets) >=
+            6 * (int64_t)num_sms())
+        h->tune.bdd_fp_cols = 16;
     if (desc->bp_type == 5 && desc->n_rows_d % 4 == 0 && desc->nz >= 16 &&
         (int64_t)((desc->nx + 31) / 32) * ((desc->ny + 3) / 4) * (desc->nz / 16) >= 5 * (int64_t)num_sms())
         h->tune.bdd_bp_z = 16;

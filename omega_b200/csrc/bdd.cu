@@ -81,21 +81,22 @@ __global__ void k_bdd_fp(Grid g, const float *__restrict__ xy, const float *__re
         // The 8 columns partition [zu, zu + 8w] along z.  With C(b) the
         // integral of the lateral row integrals from zu up to b, column c is
         // C(b_{c+1}) - C(b_c): walk b_0 < ... < b_8 and the voxel rows
-        // together, one row integral per row crossed.
+        // together, one row integral per row crossed (T: the integral up to
+        // the current row's end).
         float bz = fminf(fmaxf(zu, 0.f), fz);
         int kc = min((int)bz, zmax);
         float R = row_integral(kc);
-        float S = 0.f;
-        float Cprev = (bz - (float)kc) * R;
+        float T = R;
+        float Cprev = fmaf(bz - (float)(kc + 1), R, T);
 #pragma unroll
         for (int c = 0; c < kColsPerThread; ++c) {
             bz = fminf(fmaxf(fmaf((float)(c + 1), w, zu), 0.f), fz);
             const int kn = min((int)bz, zmax);
             while (kc < kn) {
-                S += R;
                 R = row_integral(++kc);
+                T += R;
             }
-            const float C = fmaf(bz - (float)kc, R, S);
+            const float C = fmaf(bz - (float)(kc + 1), R, T);
             temp[c] = fmaf(C - Cprev, inv_area, temp[c]);
             Cprev = C;
         }

@@ -32,10 +32,16 @@ __device__ int g_device_error = 0;
 namespace bt {
 
 constexpr int kBW = 40;       // lateral voxels of a staged box (x multiple of 4: 16-byte aligned starts)
-constexpr int kBZ = 36;       // voxel rows (z) of a staged box
-constexpr int kStages = 4;    // ring depth
-constexpr int kCTACols = 32;  // detector columns of a CTA (kCTACols / C warps of C-column groups)
-constexpr int kBoxFloats = kBW * kBZ;
+// 4 warps of C-column groups.  A slice costs a thread about 90 instructions
+// whatever its columns (footprint lines, area, run weights, the stage's wait),
+// so 16 columns share them among twice as many as 8.
+template <int C>
+struct Fp {
+    static constexpr int kCols = 4 * C;               // detector columns of a CTA
+    static constexpr int kBZ = C == 16 ? 60 : 36;     // voxel rows (z) of a staged box
+    static constexpr int kStages = C == 16 ? 3 : 4;   // ring depth
+    static constexpr int kBoxFloats = kBW * kBZ;
+};
 constexpr int kWaitTries = 1 << 22;
 constexpr int kWaitTriesAfterFailure = 64;
 
@@ -61,17 +67,22 @@ struct Corner {
     float xa0, xa1, xb0, xb1, za0, za1, zb0, zb1, dz0, dz1;
 };
 
-struct Shared {
-    alignas(128) float box[kStages][kBoxFloats];
-    alignas(8) uint64_t full[kStages];
-    int2 origin[kStages];  // (lateral, z) voxel of the box's first element
+struct Lines {
     Corner corner[4];
     int2 slices;           // [first, last] slice the CTA's rays can meet
 };
 
+template <int C>
+struct Shared {
+    alignas(128) float box[Fp<C>::kStages][Fp<C>::kBoxFloats];
+    alignas(8) uint64_t full[Fp<C>::kStages];
+    int2 origin[Fp<C>::kStages];  // (lateral, z) voxel of the box's first element
+    Lines lines;
+};
+
 // Box of slice j covering the four corner rays' footprints (lateral start
 // rounded down to a multiple of 4), clamped into the volume.
-__device__ __forceinline__ int2 slice_box(const Shared &sh, int j, int nlat, int nz) {
+__device__ __forceinline__ int2 slice_box(const Lines &sh, int j, int nlat, int nz) {
     const float fj = (float)j;
     float lo = 3.4e38f, zlo = 3.4e38f;
 #pragma unroll
@@ -97,9 +108,10 @@ __global__ void k_bdd_fp_tma(const __grid_constant__ CUtensorMap map_img, const 
                              float pitch_y, int64_t proj0, int64_t nproj, const float *__restrict__ img,
                              const float *__restrict__ imgT, float *__restrict__ y) {
     using namespace bt;
-    constexpr int kRB = kCTACols / NC;  // warps per CTA
+    constexpr int kRB = 4;  // warps per CTA
+    constexpr int kBZ = Fp<NC>::kBZ, kStages = Fp<NC>::kStages, kBoxFloats = Fp<NC>::kBoxFloats;
     constexpr float kC = (float)NC;
-    __shared__ Shared sh;
+    __shared__ Shared<NC> sh;
     const int tid = threadIdx.x + threadIdx.y * 32;
     const int r = blockIdx.x * 32 + threadIdx.x;
     const int cg = blockIdx.y * kRB + threadIdx.y;
@@ -115,7 +127,7 @@ __global__ void k_bdd_fp_tma(const __grid_constant__ CUtensorMap map_img, const 
         const int rr = (tid & 1) ? r_last : (int)blockIdx.x * 32;
         const int cc = ((tid & 2) ? g_last : (int)blockIdx.y * kRB) * NC;
         const BddRay b = bdd_ray_setup(g, xy, uv, proj0 + p, rr, cc, nr, nc, pitch_y);
-        sh.corner[tid] = Corner{b.xa0, b.xa1, b.xb0, b.xb1, b.za0, b.za1, b.zb0, b.zb1, b.dz0, b.dz1};
+        sh.lines.corner[tid] = Corner{b.xa0, b.xa1, b.xb0, b.xb1, b.za0, b.za1, b.zb0, b.zb1, b.dz0, b.dz1};
         if (tid == 0) {
             for (int s = 0; s < kStages; ++s)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&sh.full[s])) : "memory");
@@ -135,17 +147,17 @@ __global__ void k_bdd_fp_tma(const __grid_constant__ CUtensorMap map_img, const 
     if (tid == 0) {
         SliceRange range = slice_range_empty();
         for (int q = 0; q < 4; ++q) {
-            const Corner &c = sh.corner[q];
+            const Corner &c = sh.lines.corner[q];
             slice_range_add(range, c.xa0, c.xa1, c.xb0, c.xb1, c.za0, c.za1, c.zb0, c.zb1, nsl, nlat, g.nz, kC);
         }
-        sh.slices = slice_range_bounds(range);
+        sh.lines.slices = slice_range_bounds(range);
     }
     __syncthreads();
-    const int j_lo = sh.slices.x, j_hi = sh.slices.y;
+    const int j_lo = sh.lines.slices.x, j_hi = sh.lines.slices.y;
 
     // loads slice jn into stage s (one thread)
     auto issue = [&](int jn, int s) {
-        const int2 o = slice_box(sh, jn, nlat, g.nz);
+        const int2 o = slice_box(sh.lines, jn, nlat, g.nz);
         sh.origin[s] = o;
         const uint32_t bar = smem_u32(&sh.full[s]);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar),
@@ -211,47 +223,53 @@ __global__ void k_bdd_fp_tma(const __grid_constant__ CUtensorMap map_img, const 
                 // column edges to [0, nz] and of the row to nz - 1 are identities
                 const float *q = sh.box[s] + (kc - o.y) * kBW + (i0 - o.x);
                 const float *q1 = q + seg.o1, *q2 = q + seg.o2;
-                float R = fmaf(seg.w2, *q2, fmaf(seg.w1, *q1, seg.w0 * q[0]));
-                float S = 0.f;
-                // the row as an exact float: with bz >= 0 and at most one new
-                // row per column, (int)bz > kc is bz >= kc + 1, so no
-                // float-to-int conversion per column
-                float fkc = (float)kc;
-                float Cprev = (bz - fkc) * R;
+                // the row's end as an exact float: with bz >= 0 and at most one
+                // new row per column, (int)bz > kc is bz >= kb, so no
+                // float-to-int conversion per column.  T is the integral up to kb.
+                float kb = (float)(kc + 1);
+                auto columns = [&](auto row) {
+                    float R = row();
+                    float T = R;
+                    float Cprev = fmaf(bz - kb, R, T);
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    bz = fmaf((float)(c + 1), w, zu);
-                    if (bz >= fkc + 1.f) {
-                        S += R;
-                        fkc += 1.f;
-                        q += kBW;
-                        q1 += kBW;
-                        q2 += kBW;
-                        R = fmaf(seg.w2, *q2, fmaf(seg.w1, *q1, seg.w0 * q[0]));
+                    for (int c = 0; c < NC; ++c) {
+                        bz = fmaf((float)(c + 1), w, zu);
+                        if (bz >= kb) {
+                            kb += 1.f;
+                            q += kBW;
+                            q1 += kBW;
+                            q2 += kBW;
+                            R = row();
+                            T += R;
+                        }
+                        const float C = fmaf(bz - kb, R, T);
+                        temp[c] = fmaf(C - Cprev, inv_area, temp[c]);
+                        Cprev = C;
                     }
-                    const float C = fmaf(bz - fkc, R, S);
-                    temp[c] = fmaf(C - Cprev, inv_area, temp[c]);
-                    Cprev = C;
-                }
+                };
+                // (a pixel no wider than a voxel meets two of them at most; its neighbours in the warp do too)
+                if (__any_sync(__activemask(), seg.n > 1))
+                    columns([&] { return fmaf(seg.w2, *q2, fmaf(seg.w1, *q1, seg.w0 * *q)); });
+                else
+                    columns([&] { return fmaf(seg.w1, *q1, seg.w0 * *q); });
             } else if (staged && seg.n <= 2 && w < 0.99f) {
                 const float *q = sh.box[s] + (kc - o.y) * kBW + (i0 - o.x);
                 float R = fmaf(seg.w2, q[seg.o2], fmaf(seg.w1, q[seg.o1], seg.w0 * q[0]));
-                float S = 0.f;
-                // min((int)bz, zmax) > kc with bz in [0, nz] is bz >= kc + 1
-                // below the last row (the exact-float row as above)
-                float fkc = (float)kc;
-                const float fzmax = (float)zmax;
-                float Cprev = (bz - fkc) * R;
+                float T = R;
+                // min((int)bz, zmax) > kc with bz in [0, nz] is bz >= kb below
+                // the last row (the exact-float row end as above)
+                float kb = (float)(kc + 1);
+                float Cprev = fmaf(bz - kb, R, T);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     bz = fminf(fmaxf(fmaf((float)(c + 1), w, zu), 0.f), fz);
-                    if (bz >= fkc + 1.f && fkc < fzmax) {
-                        S += R;
-                        fkc += 1.f;
+                    if (bz >= kb && kb < fz) {
+                        kb += 1.f;
                         q += kBW;
                         R = fmaf(seg.w2, q[seg.o2], fmaf(seg.w1, q[seg.o1], seg.w0 * q[0]));
+                        T += R;
                     }
-                    const float C = fmaf(bz - fkc, R, S);
+                    const float C = fmaf(bz - kb, R, T);
                     temp[c] = fmaf(C - Cprev, inv_area, temp[c]);
                     Cprev = C;
                 }
@@ -261,17 +279,17 @@ __global__ void k_bdd_fp_tma(const __grid_constant__ CUtensorMap map_img, const 
 #define row_integral(k) \
     (staged ? seg_sum_shared(seg, box + (k) * kBW) : seg_sum(seg, slice + (int64_t)(k) * z_stride))
                 float R = row_integral(kc);
-                float S = 0.f;
-                float Cprev = (bz - (float)kc) * R;
+                float T = R;
+                float Cprev = fmaf(bz - (float)(kc + 1), R, T);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     bz = fminf(fmaxf(fmaf((float)(c + 1), w, zu), 0.f), fz);
                     const int kn = min((int)bz, zmax);
                     while (kc < kn) {
-                        S += R;
                         R = row_integral(++kc);
+                        T += R;
                     }
-                    const float C = fmaf(bz - (float)kc, R, S);
+                    const float C = fmaf(bz - (float)(kc + 1), R, T);
                     temp[c] = fmaf(C - Cprev, inv_area, temp[c]);
                     Cprev = C;
                 }
@@ -516,13 +534,13 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// 3-D map of a volume stored (lat, slice, z) with lat fastest; box kBW x 1 x kBZ.
-static bool encode_volume(CUtensorMap &m, const float *base, int nlat, int nsl, int nz) {
+// 3-D map of a volume stored (lat, slice, z) with lat fastest; box kBW x 1 x box_rows.
+static bool encode_volume(CUtensorMap &m, const float *base, int nlat, int nsl, int nz, int box_rows) {
     auto fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)nlat, (cuuint64_t)nsl, (cuuint64_t)nz};
     const cuuint64_t strides[2] = {(cuuint64_t)nlat * sizeof(float), (cuuint64_t)nlat * nsl * sizeof(float)};
-    const cuuint32_t box[3] = {(cuuint32_t)bt::kBW, 1u, (cuuint32_t)bt::kBZ};
+    const cuuint32_t box[3] = {(cuuint32_t)bt::kBW, 1u, (cuuint32_t)box_rows};
     const cuuint32_t estr[3] = {1u, 1u, 1u};
     return fn(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -538,10 +556,11 @@ bool bdd_fp_tma_supported(const Grid &g, const float *img, const float *imgT) {
 int bdd_forward_tma(const Grid &g, const float *xy, const float *uv, int nr, int nc, float pitch_y, int64_t proj0,
                     int64_t nproj, const float *img, const float *imgT, float *y, int cols, cudaStream_t st) {
     CUtensorMap m_img, m_imgT;
-    if (!encode_volume(m_img, img, g.nx, g.ny, g.nz) || !encode_volume(m_imgT, imgT, g.ny, g.nx, g.nz))
-        return set_error(OMB_ERR_CUDA, "cuTensorMapEncodeTiled failed for the type-5 image maps");
     const int C = cols == 16 ? 16 : 8;
-    const int rb = bt::kCTACols / C;
+    const int rows = C == 16 ? bt::Fp<16>::kBZ : bt::Fp<8>::kBZ;
+    if (!encode_volume(m_img, img, g.nx, g.ny, g.nz, rows) || !encode_volume(m_imgT, imgT, g.ny, g.nx, g.nz, rows))
+        return set_error(OMB_ERR_CUDA, "cuTensorMapEncodeTiled failed for the type-5 image maps");
+    const int rb = 4;
     const int groups = (nc + C - 1) / C;
     dim3 block(32, rb);
     dim3 grid((nr + 31) / 32, (groups + rb - 1) / rb, (unsigned)nproj);
