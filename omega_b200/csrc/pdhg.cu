@@ -133,8 +133,31 @@ __global__ void k_normalize_into(float *__restrict__ x, const float *__restrict_
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) x[i] = __ldg(b + i) * inv;
 }
 
+// Four elements per thread, no loop (94 M elements: 408 us with one at a time
+// at 4 blocks per SM; the PDHG iteration 22.55 -> 22.34 ms).
+__global__ void k_pdhg_dual4(float4 *__restrict__ p, const float4 *__restrict__ fp, const float4 *__restrict__ y,
+                             int64_t n4, float sigma) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n4) return;
+    const float inv = 1.f / (1.f + sigma);
+    const float4 f = __ldg(fp + i), m = __ldg(y + i);
+    float4 q = p[i];
+    q.x = (q.x + sigma * (f.x - m.x)) * inv;
+    q.y = (q.y + sigma * (f.y - m.y)) * inv;
+    q.z = (q.z + sigma * (f.z - m.z)) * inv;
+    q.w = (q.w + sigma * (f.w - m.w)) * inv;
+    p[i] = q;
+}
+
 int pdhg_dual(float *p, const float *fp, const float *y, int64_t n, float sigma, cudaStream_t st) {
     if (n <= 0) return OMB_OK;
+    if (n % 4 == 0 && (((uintptr_t)p | (uintptr_t)fp | (uintptr_t)y) & 15) == 0 && n / 4 / kBlock < 0x7fffffff) {
+        k_pdhg_dual4<<<(unsigned)((n / 4 + kBlock - 1) / kBlock), kBlock, 0, st>>>(
+            reinterpret_cast<float4 *>(p), reinterpret_cast<const float4 *>(fp), reinterpret_cast<const float4 *>(y),
+            n / 4, sigma);
+        OMB_LAUNCH_CHECK("pdhg dual launch");
+        return OMB_OK;
+    }
     k_pdhg_dual<<<grid_for(n, 4), kBlock, 0, st>>>(p, fp, y, n, sigma);
     OMB_LAUNCH_CHECK("pdhg dual launch");
     return OMB_OK;
