@@ -274,11 +274,33 @@ __global__ void __launch_bounds__(kBlock) k_interp_bp(Grid g, RaySet rs, Tof tof
         // rays along x add to the y-fastest image; a sample off the grid's far
         // faces in x or y lands on the x-fastest index it always had
         const bool yfast = W == 0 && !SENS && (FIXED ? accT != nullptr : imgT != nullptr) && runs_along_x(ray.s, ray.d);
+        // Most samples lie clear of every face: within kClear voxels of one the
+        // FP64 decision is made, elsewhere the FP32 position picks the same voxel
+        // at a third of the instructions, none of them on the FP64 pipe.  On
+        // grids of up to 1024 voxels per axis it is off by at most 1.3e-4 voxels
+        // (first sample 3e-5, step times index 6e-5, sum 3e-5).
+        constexpr float kClear = 2e-4f;
+        const float ox = (float)((sx + vx * m.ts - bx) * ivx), oy = (float)((sy + vy * m.ts - by) * ivy),
+                    oz = (float)((sz + vz * m.ts - bz) * ivz);
+        const bool fits = m.n < (1u << 24) && g.nx <= 1024 && g.ny <= 1024 && g.nz <= 1024;
         for (unsigned ii = 0; ii < m.n; ++ii) {
-            const double t = __dadd_rn(m.ts, __dmul_rn((double)ii, m.tstep));
-            const unsigned ux = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sx, __dmul_rn(vx, t)), bx), ivx));
-            const unsigned uy = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sy, __dmul_rn(vy, t)), by), ivy));
-            const unsigned uz = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sz, __dmul_rn(vz, t)), bz), ivz));
+            const float fi = (float)ii;
+            const float px = fmaf(fi, m.sx, ox), py = fmaf(fi, m.sy, oy), pz = fmaf(fi, m.sz, oz);
+            const float fx = __fadd_rd(px, 8388608.f), fy = __fadd_rd(py, 8388608.f), fz = __fadd_rd(pz, 8388608.f);
+            // distance past the lower face, in [0, 1] inside
+            const float rx = px - (fx - 8388608.f), ry = py - (fy - 8388608.f), rz = pz - (fz - 8388608.f);
+            unsigned ux, uy, uz;
+            if (fits && fminf(fminf(px, py), pz) > 0.f && fminf(fminf(rx, ry), rz) > kClear &&
+                fmaxf(fmaxf(rx, ry), rz) < 1.f - kClear) {
+                ux = __float_as_uint(fx) & 0x7fffffu;
+                uy = __float_as_uint(fy) & 0x7fffffu;
+                uz = __float_as_uint(fz) & 0x7fffffu;
+            } else {
+                const double t = __dadd_rn(m.ts, __dmul_rn((double)ii, m.tstep));
+                ux = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sx, __dmul_rn(vx, t)), bx), ivx));
+                uy = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sy, __dmul_rn(vy, t)), by), ivy));
+                uz = voxel_of(__dmul_rn(__dsub_rn(__dadd_rn(sz, __dmul_rn(vz, t)), bz), ivz));
+            }
             const unsigned ind = ux + uy * nx + uz * nxy;
             if (ind == 0u || ind >= ntot) continue;
             float yax, val;
@@ -359,6 +381,34 @@ __global__ void k_interp_ct_bp(Grid g, const BddProj *__restrict__ pj, int nr, i
         const float vx = qx - P.s[0], vy = qy - P.s[1];
         const float axy = fmaf(vx, vx, vy * vy);
         const float *yp = y + p * (int64_t)nr * nc;
+        // Panels whose columns run along z (every panel of the geometry code):
+        // the row coordinate and the distance are those of the whole run, and
+        // a run that lands inside the panel needs no clamps: 31 instructions
+        // per voxel and view instead of about 60 (170 x 170 x 121, 90 views
+        // forward and back: 3.86 -> 3.45 ms).
+        if (!SENS && su == 0.f && sd == 0.f && nzt == kCtZ) {
+            const float inv = 1.f / de0;
+            const float u = nu0 * inv - 0.5f, va = nv0 * inv - 0.5f, vb = fmaf((float)(kCtZ - 1), sv, nv0) * inv - 0.5f;
+            // (margins far above the rounding of the coordinates)
+            if (u >= 0.01f && u < fnr - 1.01f && fminf(va, vb) >= 0.01f && fmaxf(va, vb) < fnc - 1.01f) {
+                const float big = 8388608.f;
+                const float tu = __fadd_rd(u, big), au = u - (tu - big);
+                const float *row = yp + (__float_as_int(tu) & 0x7fffff);
+                const float tt = P.k * inv, scale = tt * tt * tt;
+#pragma unroll
+                for (int t = 0; t < kCtZ; ++t) {
+                    const float ft = (float)t;
+                    const float v = fmaf(ft, sv, nv0) * inv - 0.5f;
+                    const float tv = __fadd_rd(v, big), av = v - (tv - big);
+                    const float *q = row + (int64_t)(__float_as_int(tv) & 0x7fffff) * nr, *q1 = q + nr;
+                    const float a = __ldg(q), b = __ldg(q + 1), c = __ldg(q1), d = __ldg(q1 + 1);
+                    const float e0 = fmaf(au, b - a, a), e1 = fmaf(au, d - c, c);
+                    const float vz = fmaf(ft, g.dz, qz0) - P.s[2];
+                    temp[t] = fmaf(fmaf(av, e1 - e0, e0), sqrtf(fmaf(vz, vz, axy)) * scale * kerroin, temp[t]);
+                }
+                continue;
+            }
+        }
 #pragma unroll
         for (int t = 0; t < kCtZ; ++t) {
             if (t < nzt) {
