@@ -197,7 +197,7 @@ struct Tuning {
     int siddon_blocks_per_sm = 8;   // grid-stride grid of the Siddon kernels: blocks per SM
     int siddon_frames = 8;          // most frames sharing one ray walk (1, 2, 4, 8)
     int bdd_fp_cols = 8;            // type-5 forward: detector columns per thread (8, 16)
-    int bdd_bp_z = 8;               // type-5 backward: voxels along z per thread (4, 8, 16; 16 from the start for volumes that fill the chip with it)
+    int bdd_bp_z = 8;               // type-5 backward: voxels along z per thread (4, 8, 16)
     int bdd_fp_rows = 8;            // type-5 forward: warps per block (4, 8)
     int bdd_bp_rows = 8;            // type-5 backward: warps per block (4, 8)
     int siddon_layout = 1;          // frame batches: 0 = frame-major reads/atomics, 1 = voxel-interleaved
@@ -255,6 +255,18 @@ inline unsigned grid_for(int64_t n, int per_sm = 8, int block = kBlock) {
     int64_t cap = (int64_t)num_sms() * per_sm;
     if (need < 1) need = 1;
     return (unsigned)(need < cap ? need : cap);
+}
+
+// Threads per block of a kernel with one ray per thread.  Few rays (up to two
+// full sets of resident threads): blocks of 64, so that the last ones spread
+// over the SMs evenly (80,352 rays are 314 blocks of 256, 2 or 3 on an SM, but
+// 1,256 of 64, 8 or 9).  One subset forward and back: 80,352 rays 87 -> 82 us,
+// 378,432 rays of type 4 280 -> 264 us, 472,080 TOF rays 1.38 -> 1.32 ms.
+inline int ray_block(int64_t rays) { return rays < (int64_t)num_sms() * 2 * 2048 ? 64 : kBlock; }
+// `per_sm`: blocks of kBlock threads per SM at most
+inline unsigned ray_grid(int64_t rays, int per_sm) {
+    const int block = ray_block(rays);
+    return grid_for(rays, per_sm * (kBlock / block), block);
 }
 
 }  // namespace omb

@@ -442,7 +442,7 @@ __global__ void k_interp_ct_bp(Grid g, const BddProj *__restrict__ pj, int nr, i
 int interp_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, float dL, const float *img,
                    const __nv_bfloat16 *img16, float *y, const Tuning &tn, cudaStream_t st) {
     if (rs.m_size <= 0) return OMB_OK;
-    const unsigned grid = grid_for(rs.m_size, tn.siddon_blocks_per_sm);
+    const unsigned grid = ray_grid(rs.m_size, tn.siddon_blocks_per_sm);
     const size_t vox = img16 ? sizeof(__nv_bfloat16) : sizeof(float);
     const StreamScratch copy(tof.nbins == 1 && orient_pays(g, rs) ? (size_t)g.nx * g.ny * g.nz * vox : 0, st);
     if (copy.p) {
@@ -454,10 +454,10 @@ int interp_forward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, fl
 #define X(n)                                                                                    \
     case n:                                                                                     \
         if (img16)                                                                              \
-            k_interp_fp<n, __nv_bfloat16><<<grid, kBlock, 0, st>>>(                             \
+            k_interp_fp<n, __nv_bfloat16><<<grid, ray_block(rs.m_size), 0, st>>>(                             \
                 g, rs, tof, gf, dL, img16, static_cast<const __nv_bfloat16 *>(copy.p), y);      \
         else                                                                                    \
-            k_interp_fp<n, float><<<grid, kBlock, 0, st>>>(                                     \
+            k_interp_fp<n, float><<<grid, ray_block(rs.m_size), 0, st>>>(                                     \
                 g, rs, tof, gf, dL, img, static_cast<const float *>(copy.p), y);                \
         break;
         X(0)
@@ -476,13 +476,13 @@ static void bp_launch4(unsigned grid, const Grid &g, const RaySet &rs, const Tof
                        unsigned long long *accT, unsigned long long *acc_s, cudaStream_t st) {
     if (acc) {
         if (acc_s)
-            k_interp_bp<W, true, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
+            k_interp_bp<W, true, true><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
         else
-            k_interp_bp<W, false, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
+            k_interp_bp<W, false, true><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
     } else if (sens) {
-        k_interp_bp<W, true, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
+        k_interp_bp<W, true, false><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
     } else {
-        k_interp_bp<W, false, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
+        k_interp_bp<W, false, false><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, dL, y, img, imgT, sens, acc, accT, acc_s);
     }
 }
 
@@ -492,7 +492,7 @@ int interp_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, f
     if (rs.m_size <= 0) return OMB_OK;
     if ((uint64_t)g.nx * g.ny * g.nz >= (1ull << 32))
         return set_error(OMB_ERR_UNSUPPORTED, "type-4 backprojection needs fewer than 2^32 voxels");
-    const unsigned grid = grid_for(rs.m_size, tn.siddon_blocks_per_sm);
+    const unsigned grid = ray_grid(rs.m_size, tn.siddon_blocks_per_sm);
     // rays along x add to a y-fastest image of their own, added to the result at the end
     const size_t bytes = (size_t)g.nx * g.ny * g.nz * (acc ? sizeof(unsigned long long) : sizeof(float));
     const StreamScratch along_x(!sens && !acc_s && (acc || img) && tof.nbins == 1 && orient_pays(g, rs) ? bytes : 0, st);

@@ -423,13 +423,13 @@ __global__ void k_fixed_to_float(const unsigned long long *__restrict__ acc, flo
 template <int FB, int K>
 static void fp_launch_k(const Grid &g, const RaySet &rs, float gf, const Frames &fr, const void *imgT, int per_sm,
                         cudaStream_t st) {
-    dim3 grid(grid_for(rs.m_size, per_sm), (fr.n + FB - 1) / FB);
+    dim3 grid(ray_grid(rs.m_size, per_sm), (fr.n + FB - 1) / FB);
     if (fr.img_in16)
-        k_siddon_fp<FB, __nv_bfloat16, K><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.img_in16,
+        k_siddon_fp<FB, __nv_bfloat16, K><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, gf, fr.img_in16,
                                                                    static_cast<const __nv_bfloat16 *>(imgT), fr.img_stride,
                                                                    fr.meas_out, fr.meas_stride, fr.n);
     else
-        k_siddon_fp<FB, float, K><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.img_in, static_cast<const float *>(imgT),
+        k_siddon_fp<FB, float, K><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, gf, fr.img_in, static_cast<const float *>(imgT),
                                                            fr.img_stride, fr.meas_out, fr.meas_stride, fr.n);
 }
 
@@ -445,38 +445,38 @@ static void fp_launch(const Grid &g, const RaySet &rs, float gf, const Frames &f
 template <int FB>
 static void bp_launch(const Grid &g, const RaySet &rs, float gf, const Frames &fr, float *imgT, float *sens,
                       int per_sm, cudaStream_t st) {
-    dim3 grid(grid_for(rs.m_size, per_sm), (fr.n + FB - 1) / FB);
+    dim3 grid(ray_grid(rs.m_size, per_sm), (fr.n + FB - 1) / FB);
     if (sens)
-        k_siddon_bp<FB, true><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, nullptr, fr.img_stride,
+        k_siddon_bp<FB, true><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, nullptr, fr.img_stride,
                                                        sens, fr.n);
     else
-        k_siddon_bp<FB, false><<<grid, kBlock, 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, imgT, fr.img_stride,
+        k_siddon_bp<FB, false><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, gf, fr.meas, fr.meas_stride, fr.img, imgT, fr.img_stride,
                                                         nullptr, fr.n);
 }
 
 template <int W>
 static void fp_tof_launch(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const Frames &fr, int per_sm,
                           cudaStream_t st) {
-    const unsigned grid = grid_for(rs.m_size, per_sm);
+    const unsigned grid = ray_grid(rs.m_size, per_sm);
     if (fr.img_in16)
-        k_siddon_fp_tof<W, __nv_bfloat16><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, fr.img_in16, fr.meas_out);
+        k_siddon_fp_tof<W, __nv_bfloat16><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, fr.img_in16, fr.meas_out);
     else
-        k_siddon_fp_tof<W, float><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, fr.img_in, fr.meas_out);
+        k_siddon_fp_tof<W, float><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, fr.img_in, fr.meas_out);
 }
 
 template <int W>
 static void bp_tof_launch(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const float *y, float *img,
                           float *sens, unsigned long long *acc, unsigned long long *acc_sens, int per_sm,
                           cudaStream_t st) {
-    const unsigned grid = grid_for(rs.m_size, per_sm);
+    const unsigned grid = ray_grid(rs.m_size, per_sm);
     if (acc && acc_sens)
-        k_siddon_bp_tof<W, true, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
+        k_siddon_bp_tof<W, true, true><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
     else if (acc)
-        k_siddon_bp_tof<W, false, true><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
+        k_siddon_bp_tof<W, false, true><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
     else if (sens)
-        k_siddon_bp_tof<W, true, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
+        k_siddon_bp_tof<W, true, false><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
     else
-        k_siddon_bp_tof<W, false, false><<<grid, kBlock, 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
+        k_siddon_bp_tof<W, false, false><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, tof, gf, y, img, sens, acc, acc_sens);
 }
 
 // Frames per walk for non-TOF batches (at most `most`).
@@ -608,12 +608,12 @@ int siddon_backward_fixed(const Grid &g, const RaySet &rs, const Tof &tof, float
     const StreamScratch along_x(may_allocate && !acc_sens && tof.nbins == 1 && orient_pays(g, rs) ? bytes : 0, st);
     auto *accT = static_cast<unsigned long long *>(along_x.p);
     if (accT) OMB_CUDA_TRY(cudaMemsetAsync(accT, 0, bytes, st));
-    const unsigned grid = grid_for(rs.m_size);
+    const unsigned grid = ray_grid(rs.m_size, 8);
     if (tof.nbins == 1) {
         if (acc_sens)
-            k_siddon_bp_fixed<true><<<grid, kBlock, 0, st>>>(g, rs, gf, y, acc, nullptr, acc_sens);
+            k_siddon_bp_fixed<true><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, gf, y, acc, nullptr, acc_sens);
         else
-            k_siddon_bp_fixed<false><<<grid, kBlock, 0, st>>>(g, rs, gf, y, acc, accT, nullptr);
+            k_siddon_bp_fixed<false><<<grid, ray_block(rs.m_size), 0, st>>>(g, rs, gf, y, acc, accT, nullptr);
     } else {
         // every bin in the window, in the given order: callers that hold the
         // centres on the device only (omb_backward_fixed64_noalloc) cannot have
