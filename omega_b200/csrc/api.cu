@@ -1034,13 +1034,19 @@ int omb_osem_subset_frames(omb_handle *h, int32_t subset, int32_t n_frames, floa
     else
         st = osem_ratio_frames(y_subset, y_stride, work_meas, m, m, n_frames, eps, s);
     if (st != OMB_OK) return st;
-    OMB_CUDA_TRY(cudaMemsetAsync(work_img, 0, (size_t)n_frames * h->n_img * sizeof(float), s));
     Frames b{};
     b.n = n_frames;
     b.meas = work_meas;
     b.meas_stride = m;
     b.img = work_img;
     b.img_stride = h->n_img;
+    if (h->desc.bp_type == 1 && !h->tune.siddon_bp_matrix && rs.nr_xy * rs.nr_z == 1) {
+        attach_interleave(h, b, s);
+        st = siddon_backward_em(h->grid, rs, h->tof, h->desc.global_factor, b, h->tune,
+                                EmFrames{sens, images, image_stride, eps}, s);
+        if (st != 1) return st;
+    }
+    OMB_CUDA_TRY(cudaMemsetAsync(work_img, 0, (size_t)n_frames * h->n_img * sizeof(float), s));
     st = rays_backward(h, rs, b, nullptr, s);
     if (st != OMB_OK) return st;
     return em_update_frames(images, image_stride, sens, work_img, h->n_img, h->n_img, n_frames, eps, s);

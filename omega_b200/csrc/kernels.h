@@ -12,6 +12,17 @@ int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, c
 // may_allocate: the call may take scratch memory
 int siddon_backward_fixed(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const float *y,
                           unsigned long long *acc, unsigned long long *acc_sens, bool may_allocate, cudaStream_t st);
+// Backprojection of a frame batch and its EM update (img: the frames' images,
+// `stride` apart) in one go, from the interleaved sums; 1 when the batch does
+// not take the interleaved kernels (nothing was done).
+struct EmFrames {
+    const float *sens;
+    float *img;
+    int64_t stride;
+    float epps;
+};
+int siddon_backward_em(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const Frames &fr, const Tuning &tn,
+                       const EmFrames &em, cudaStream_t st);
 // y-fastest copy of an image, and the sum of one into an image (oriented images, common.cuh)
 int transpose_xy(const Grid &g, const float *in, float *out, cudaStream_t st);
 int transpose_xy(const Grid &g, const __nv_bfloat16 *in, __nv_bfloat16 *out, cudaStream_t st);

@@ -157,6 +157,37 @@ __global__ void __launch_bounds__(kBlock) k_frames_deinterleave(const float *__r
     }
 }
 
+// The EM update of a batch straight from the interleaved backprojection: x = x
+// / sens * (rhs + epps) without writing the images of rhs out and reading them
+// back (24 frames of 128 x 128 x 63, 16 subsets: 15.9 -> 15.1 ms per iteration).
+template <int FB>
+__global__ void __launch_bounds__(kBlock) k_em_update_ilv(const float *__restrict__ rhs, const float *__restrict__ sens,
+                                                          int n_frames, int64_t n, float *__restrict__ img,
+                                                          int64_t img_stride, float epps) {
+    const int f0 = blockIdx.y * FB;
+    const int nf = min(FB, n_frames - f0);
+    const float4 *p = reinterpret_cast<const float4 *>(rhs + (int64_t)blockIdx.y * n * FB);
+    img += f0 * img_stride;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+        float a[FB], x[FB];
+        const float s = __ldg(sens + v);
+#pragma unroll
+        for (int f = 0; f < FB; ++f) x[f] = f < nf ? img[f * img_stride + v] : 0.f;
+#pragma unroll
+        for (int q = 0; q < FB / 4; ++q) {
+            const float4 t = __ldg(p + v * (FB / 4) + q);
+            a[4 * q] = t.x;
+            a[4 * q + 1] = t.y;
+            a[4 * q + 2] = t.z;
+            a[4 * q + 3] = t.w;
+        }
+#pragma unroll
+        for (int f = 0; f < FB; ++f)
+            if (f < nf) img[f * img_stride + v] = x[f] / s * (a[f] + epps);
+    }
+}
+
 template <int FB, int K>
 __global__ void __launch_bounds__(kBlock, 4) k_siddon_fp_ilv(Grid g, RaySet rs, float gf, const float *__restrict__ img,
                                                           int64_t n_img, float *__restrict__ y, int64_t y_stride,
@@ -512,11 +543,16 @@ static void fp_ilv_launch(const Grid &g, const RaySet &rs, float gf, const Frame
 
 template <int FB>
 static int bp_ilv_launch(const Grid &g, const RaySet &rs, float gf, const Frames &fr, int64_t n_img, int per_sm,
-                         cudaStream_t st) {
+                         const EmFrames *em, cudaStream_t st) {
     const unsigned groups = (fr.n + FB - 1) / FB;
     OMB_CUDA_TRY(cudaMemsetAsync(fr.ilv, 0, (size_t)groups * FB * n_img * sizeof(float), st));
     k_siddon_bp_ilv<FB><<<dim3(grid_for(rs.m_size, per_sm), groups), kBlock, 0, st>>>(g, rs, gf, fr.meas,
                                                                                         fr.meas_stride, fr.ilv, n_img, fr.n);
+    if (em) {
+        k_em_update_ilv<FB><<<dim3(grid_for(n_img, 16), groups), kBlock, 0, st>>>(fr.ilv, em->sens, fr.n, n_img, em->img,
+                                                                                  em->stride, em->epps);
+        return OMB_OK;
+    }
     k_frames_deinterleave<FB><<<dim3(grid_for(n_img, 4), groups), kBlock, 0, st>>>(fr.ilv, fr.n, n_img, fr.img,
                                                                                     fr.img_stride);
     return OMB_OK;
@@ -576,10 +612,10 @@ int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, c
     float *imgT = static_cast<float *>(along_x.p);
     if (imgT) OMB_CUDA_TRY(cudaMemsetAsync(imgT, 0, n_img * sizeof(float), st));
     if (ilv == 8) {
-        const int e = bp_ilv_launch<8>(g, rs, gf, fr, n_img, ps, st);
+        const int e = bp_ilv_launch<8>(g, rs, gf, fr, n_img, ps, nullptr, st);
         if (e != OMB_OK) return e;
     } else if (ilv == 4) {
-        const int e = bp_ilv_launch<4>(g, rs, gf, fr, n_img, ps, st);
+        const int e = bp_ilv_launch<4>(g, rs, gf, fr, n_img, ps, nullptr, st);
         if (e != OMB_OK) return e;
     } else if (tof.nbins == 1) {
         switch (frames_per_walk(fr.n, tn.siddon_frames)) {
@@ -599,6 +635,18 @@ int siddon_backward(const Grid &g, const RaySet &rs, const Tof &tof, float gf, c
     }
     OMB_LAUNCH_CHECK("siddon backward launch");
     return imgT ? add_transposed(g, imgT, fr.img, st) : OMB_OK;
+}
+
+int siddon_backward_em(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const Frames &fr, const Tuning &tn,
+                       const EmFrames &em, cudaStream_t st) {
+    const int64_t n_img = (int64_t)g.nx * g.ny * g.nz;
+    const int ilv = rs.m_size > 0 ? interleaved_frames(tof, fr, tn, n_img) : 0;
+    if (ilv == 0) return 1;
+    const int e = ilv == 8 ? bp_ilv_launch<8>(g, rs, gf, fr, n_img, tn.siddon_blocks_per_sm, &em, st)
+                           : bp_ilv_launch<4>(g, rs, gf, fr, n_img, tn.siddon_blocks_per_sm, &em, st);
+    if (e != OMB_OK) return e;
+    OMB_LAUNCH_CHECK("siddon backward and EM update launch");
+    return OMB_OK;
 }
 
 int siddon_backward_fixed(const Grid &g, const RaySet &rs, const Tof &tof, float gf, const float *y,
