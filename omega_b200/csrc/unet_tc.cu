@@ -20,7 +20,7 @@
 // Warps: 0 issues instructions, 1-3 load, 4-7 store results.  Before this a CTA
 // staged 27 tap-shifted copies of 128 voxels through registers, one
 // instruction per pair of barriers: 32 -> 32 channels at 62 x 58 x 31 x 4 took
-// 197 us, now 89.
+// 197 us, now 69.
 //
 // Every wait is bounded; on a timeout the CTA raises the error flag read by
 // omb_unet_take_error(), waits (bounded) for its copies and instructions in
@@ -124,9 +124,21 @@ struct ConvPlan {
 
 namespace tc {
 
-__device__ __forceinline__ uint64_t desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)((lbo >> 4) & 0x3FFF) << 16 |
-           (uint64_t)((sbo >> 4) & 0x3FFF) << 32 | (uint64_t)1 << 46;
+// One instruction with descriptors given as their low words (`hi` is the same
+// for both operands), issued by the lanes where `on` is set.  The whole warp
+// computes the operands: they stay in uniform registers, which the instruction
+// reads; a lone thread's would be moved there one by one.
+__device__ __forceinline__ void mma_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                       uint32_t acc, uint32_t on) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %3};\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "setp.ne.b32 e, %6, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}\n"
+        ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(acc), "r"(on)
+        : "memory");
 }
 
 }  // namespace tc
@@ -147,7 +159,7 @@ __global__ void __launch_bounds__(256) k_conv3d_tc(const __grid_constant__ ConvP
     __shared__ __align__(8) uint64_t full[4], empty[4], done, drained;
     __shared__ uint32_t tmem_base;
     __shared__ int failed;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int co0 = blockIdx.y * CO;
     if (tid == 0) {
         for (int i = 0; i < 4; ++i) {
@@ -256,41 +268,53 @@ __global__ void __launch_bounds__(256) k_conv3d_tc(const __grid_constant__ ConvP
             for (int i = total > lag ? total - lag : 0; i < total; ++i) hand_over(i);
         else if (lane == 0)
             fail();
-    } else if (tid == 0) {
+    } else if (warp == 0) {
+        const uint32_t t0 = __shfl_sync(0xffffffffu, tmem, 0), on = lane == 0;
+        // descriptor words: start address and K-half stride below, 8-row stride (128 bytes) and version above
+        constexpr uint32_t kHi = (128u >> 4) | (1u << 14);
+        const uint32_t a_base = ((ring >> 4) & 0x3FFF) | (uint32_t)(pl.plane >> 4) << 16;
+        const uint32_t b_base = ((wbase >> 4) & 0x3FFF) | (uint32_t)(3 * CO) << 16;
+        const uint32_t dstep = pl.TZ * CO;
         int it = 0;
         bool ok = true;
         for (int k = 0; k < mine && ok; ++k) {
             // the previous block's sums have been read
-            if (k > 0) ok = tc::mbar_wait(tc::smem_u32(&drained), (uint32_t)(k - 1) & 1u);
+            if (k > 0) ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&drained), (uint32_t)(k - 1) & 1u));
             for (int st = 0; st < nst && ok; ++st, ++it) {
                 const int slot = it % pl.ring;
-                ok = tc::mbar_wait(tc::smem_u32(&full[slot]), (uint32_t)(it / pl.ring) & 1u);
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&full[slot]), (uint32_t)(it / pl.ring) & 1u));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const int zr = st / NCH, c = st - zr * NCH;               // input plane z0 + zr - 1
                 const int lo = max(zr - 2, 0), hi = min(zr, pl.TZ - 1);   // output planes it adds to
                 const bool opens = c == 0 && zr < pl.TZ;                  // the last of them gets its first sum
-                const uint32_t a0 = ring + slot * pl.stage;
-                for (int t9 = 0; t9 < 9; ++t9) {
-                    const uint32_t a = a0 + (uint32_t)((t9 / 3) * pl.P + t9 % 3) * 16u;
-                    const uint32_t bw = wbase + (uint32_t)(c * 9 + t9) * WBLOCK;
-                    const uint32_t b = bw + (uint32_t)((lo - (zr - 2)) * CO) * 16u;
-                    const bool first = opens && t9 == 0;
-                    const int n = (hi - lo + 1 - (first ? 1 : 0)) * CO;
+                const uint32_t a0 = a_base + (uint32_t)(slot * (pl.stage >> 4));
+                const uint32_t b0 = b_base + (uint32_t)(c * 9 * (WBLOCK / 16)), d0 = t0 + lo * CO;
+                const uint32_t skip = (uint32_t)((lo - (zr - 2)) * CO);   // weight rows of planes below the block
+                if (opens) {
+                    // the first tap apart: it overwrites the new plane's sums and adds to the others'
+                    const int n = (hi - lo) * CO;
                     for (int t = 0; t < pl.T; ++t) {
-                        const uint64_t da = tc::desc(a + (uint32_t)(t * pl.S) * 16u, pl.plane, 128);
-                        const uint32_t d = tmem + (uint32_t)((t * pl.TZ + lo) * CO);
-                        if (n > 0) tc::mma_issue(d, da, tc::desc(b, 3 * CO * 16, 128), tc::instr_desc(n), 1u);
-                        if (first)
-                            tc::mma_issue(tmem + (uint32_t)((t * pl.TZ + hi) * CO), da,
-                                          tc::desc(bw + 2 * CO * 16, 3 * CO * 16, 128), tc::instr_desc(CO), 0u);
+                        if (n > 0)
+                            tc::mma_lo(d0 + t * dstep, a0 + t * pl.S, b0 + skip, kHi, tc::instr_desc(n), 1u, on);
+                        tc::mma_lo(t0 + hi * CO + t * dstep, a0 + t * pl.S, b0 + 2 * CO, kHi, tc::instr_desc(CO), 0u, on);
                     }
                 }
-                tc::mma_commit(tc::smem_u32(&empty[slot]));
+                const uint32_t idesc = tc::instr_desc((hi - lo + 1) * CO);
+                for (int t9 = opens ? 1 : 0; t9 < 9; ++t9) {
+                    uint32_t a = a0 + (uint32_t)(t9 / 3 * pl.P + t9 % 3), d = d0;
+                    const uint32_t b = b0 + skip + (uint32_t)(t9 * (WBLOCK / 16));
+#pragma unroll 4
+                    for (int t = 0; t < pl.T; ++t, a += pl.S, d += dstep) tc::mma_lo(d, a, b, kHi, idesc, 1u, on);
+                }
+                if (on) tc::mma_commit(tc::smem_u32(&empty[slot]));
             }
             // (on failure too: whoever waits for it is let go once the instructions in flight have ended)
-            if (!ok) fail();
-            tc::mma_commit(tc::smem_u32(&done));
+            if (on) {
+                if (!ok) fail();
+                tc::mma_commit(tc::smem_u32(&done));
+            }
+            __syncwarp();
         }
     } else if (warp >= 4) {
         const int quarter = warp & 3;   // the tensor-memory lanes this warp can read
