@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUT>::kThreads, 1)
     }
     // ldmatrix rows of this lane: matrix mi, row rr
     const int mi = lane >> 3, rr = lane & 7;
-    const int steps = pl.TX / 16, total = steps * pl.TY;
+    const int total = pl.TX / 16 * pl.TY;
     for (int k = 0; k < mine; ++k) {
         if (pl.ring == 3)
             asm volatile("cp.async.wait_group 1;\n" ::: "memory");
@@ -265,26 +265,53 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUT>::kThreads, 1)
         // input: matrices (voxels 0-7 / 8-15) of two channel planes; dz: two planes for each half of the voxels
         const uint32_t ib = st + (ns * NTW + (mi >> 1)) * pl.in_plane + ((mi & 1) * 8 + rr) * 16;
         const uint32_t db = st + pl.dz_off + (ms * MTW * 2 + (mi & 1)) * pl.dz_plane + ((mi >> 1) * 8 + rr) * 16;
-        for (int s = ks; s < total; s += S::KS) {
-            const int line = s / steps, x = (s - line * steps) * 16;
-            const uint32_t ia = ib + (uint32_t)((line + dy) * pl.TX + x) * 16u;
-            const uint32_t da = db + (uint32_t)(line * P + x) * 16u;
-            uint32_t bq[NTW / 2][4];
-#pragma unroll
-            for (int n = 0; n < NTW / 2; ++n) ldmatrix_x4_trans(bq[n], ia + 2 * n * pl.in_plane);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                // tap dx = d - 1 pairs input voxel u with dz voxel u - dx, staged at u - dx + 1
-                uint32_t aq[MTW][4];
-#pragma unroll
-                for (int m = 0; m < MTW; ++m) ldmatrix_x4_trans(aq[m], da + (2 - d) * 16 + 2 * m * pl.dz_plane);
-#pragma unroll
-                for (int m = 0; m < MTW; ++m)
-#pragma unroll
-                    for (int n = 0; n < NTW; ++n)
-                        mma_bf16(acc[d][m][n], aq[m][0], aq[m][1], aq[m][2], aq[m][3], bq[n / 2][(n & 1) * 2],
-                                 bq[n / 2][(n & 1) * 2 + 1]);
+        // two groups of 16 voxels at a time: the operands of the second are on
+        // their way while the first's are multiplied
+        int line = 0, x = ks * 16;
+        auto next = [&](uint32_t &ia, uint32_t &da) {
+            while (x >= pl.TX) {
+                x -= pl.TX;
+                ++line;
             }
+            ia = ib + (uint32_t)((line + dy) * pl.TX + x) * 16u;
+            da = db + (uint32_t)(line * P + x) * 16u;
+            x += S::KS * 16;
+        };
+        constexpr int G = MTW * NTW * 12 <= 72 ? 2 : 1;   // (registers)
+        for (int s = ks; s < total; s += G * S::KS) {
+            const bool two = G > 1 && s + S::KS < total;
+            uint32_t ia[G], da[G], bq[G][NTW / 2][4];
+            next(ia[0], da[0]);
+            if (two) next(ia[G - 1], da[G - 1]);
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (u == 0 || two) {
+#pragma unroll
+                    for (int n = 0; n < NTW / 2; ++n) ldmatrix_x4_trans(bq[u][n], ia[u] + 2 * n * pl.in_plane);
+                }
+            uint32_t aq[G][3][MTW][4];
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (u == 0 || two) {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+#pragma unroll
+                        for (int m = 0; m < MTW; ++m)
+                            // tap dx = d - 1 pairs input voxel u with dz voxel u - dx, staged at u - dx + 1
+                            ldmatrix_x4_trans(aq[u][d][m], da[u] + (2 - d) * 16 + 2 * m * pl.dz_plane);
+                }
+#pragma unroll
+            for (int u = 0; u < G; ++u)
+                if (u == 0 || two) {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+#pragma unroll
+                        for (int m = 0; m < MTW; ++m)
+#pragma unroll
+                            for (int n = 0; n < NTW; ++n)
+                                mma_bf16(acc[d][m][n], aq[u][d][m][0], aq[u][d][m][1], aq[u][d][m][2], aq[u][d][m][3],
+                                         bq[u][n / 2][(n & 1) * 2], bq[u][n / 2][(n & 1) * 2 + 1]);
+                }
         }
         // sums of at most about 8192 voxels are added up before they go to memory
         if ((k + 1) % pl.flush == 0 && k + 1 < mine) {
