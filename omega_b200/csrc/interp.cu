@@ -191,13 +191,25 @@ __global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof 
         const int nxy = g.nx * g.ny;
         auto sample = [&](float fi) {
             const float x = fmaf(fi, m.sx, m.cx), y = fmaf(fi, m.sy, m.cy), z = fmaf(fi, m.sz, m.cz);
-            return dL * (fi >= in_lo && fi <= in_hi ? trilinear_inside(im, gr.nx, nxy, x, y, z)
-                                                    : trilinear(im, gr, x, y, z));
+            return fi >= in_lo && fi <= in_hi ? trilinear_inside(im, gr.nx, nxy, x, y, z) : trilinear(im, gr, x, y, z);
         };
         if constexpr (W == 0) {
-            float ax = 0.f;
-            for (unsigned ii = 0; ii < m.n; ++ii) ax += sample((float)ii);
-            y[r] = ax * temp;
+            // the samples inside the image two at a time: sixteen loads in
+            // flight per thread instead of eight (CT, 301 x 218 x 90 rays, 170 x
+            // 170 x 121, forward and back 3.45 -> 2.78 ms; 378,432 PET rays with
+            // BF16 reads 266 -> 243 us)
+            float ax = 0.f, bx = 0.f;
+            unsigned ii = 0;
+            const unsigned lo = in_hi < in_lo ? m.n : (unsigned)fminf(in_lo, (float)m.n);
+            const unsigned hi = in_hi < in_lo ? m.n : min((unsigned)fminf(in_hi, 4e9f) + 1u, m.n);
+            for (; ii < lo; ++ii) ax += sample((float)ii);
+            for (; ii + 1 < hi; ii += 2) {
+                const float fi = (float)ii, fj = (float)(ii + 1);
+                ax += trilinear_inside(im, gr.nx, nxy, fmaf(fi, m.sx, m.cx), fmaf(fi, m.sy, m.cy), fmaf(fi, m.sz, m.cz));
+                bx += trilinear_inside(im, gr.nx, nxy, fmaf(fj, m.sx, m.cx), fmaf(fj, m.sy, m.cy), fmaf(fj, m.sz, m.cz));
+            }
+            for (; ii < m.n; ++ii) ax += sample((float)ii);
+            y[r] = (ax + bx) * dL * temp;
         } else {
             TofWindow<W> win;
             win.begin(tof, sgnf(m.D0));
@@ -205,7 +217,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_interp_fp(Grid g, RaySet rs, Tof 
             auto put = [&](int j, float v) { y[r + win.slot(tof, j) * rs.m_size] = v; };
             for (unsigned ii = 0; ii < m.n; ++ii) {
                 const float fi = (float)ii;
-                const float val = sample(fi);
+                const float val = dL * sample(fi);
                 const float p = fmaf(fi, dp, p0);
                 while (p > win.th) {
                     put(win.k, win.a[0] * temp);
