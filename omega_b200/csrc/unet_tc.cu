@@ -384,6 +384,289 @@ __global__ void __launch_bounds__(256) k_conv3d_tc(const __grid_constant__ ConvP
     }
 }
 
+// ---------------------------------------------------------------------------
+// Lines of 65 to 128 voxels.  An instruction of M = 128, K = 16 takes about 128
+// clocks whatever its N up to 256 (it reads A at 32 bytes a clock; timed with N =
+// 16 to 144), so the taps of an input line should share as few instructions as
+// their outputs allow.  A CTA marches along y with 16 output channels: for every
+// input line and dx one instruction of N = 144 columns adds to the nine output
+// lines of its (dy, dz) neighbourhood.  Their accumulators are neighbouring
+// tensor-memory columns: z planes of the block outside, three slots inside, the
+// slot of an output line its y modulo 3.  The order of the dy taps within the
+// instruction turns with y, so the weights are kept in three orders.  When an
+// input line has been added, the output line behind it is complete: it is stored
+// and its slot cleared before the next input line.  Two CTAs on an SM hide that
+// from the tensor core.  Against the kernel above (N = 3 cout, nine instructions
+// per line), 128 x 128 x 64 x 4: 16 -> 16 channels 255 to 149 us, 48 -> 16 705 to
+// 515 us, 16 -> 48 365 to 361 us; a training step of the two-level network 8.10 to
+// 7.24 ms.
+// ---------------------------------------------------------------------------
+struct LinePlan {
+    int X, Y, Z, B;
+    int TX, TZ, YS;       // x voxels, z planes and output lines of a block
+    int P;                // staged line length
+    int ntx, ntz, nys;    // blocks per axis
+    int tiles;
+    int ring, plane, stage;   // stages; bytes of an 8-channel half and of a stage
+    int cols, smem, occ;
+};
+
+template <int CIN, int COUT, bool RELU, bool MASK>
+__global__ void __launch_bounds__(256) k_conv3d_lines(const __grid_constant__ LinePlan pl,
+                                                      const __nv_bfloat16 *__restrict__ in,
+                                                      const __nv_bfloat16 *__restrict__ w,
+                                                      const float *__restrict__ bias, __nv_bfloat16 *__restrict__ out,
+                                                      const __nv_bfloat16 *__restrict__ mask) {
+    constexpr int CO = 16, NCH = CIN / 16;
+    constexpr int WBLOCK = 9 * CO * 32;            // weights of one (order, chunk, dx): 9 (dz, dy) x CO rows x 16 channels
+    constexpr int WBYTES = 3 * NCH * 3 * WBLOCK;
+    constexpr int kLoaders = 96;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(8) uint64_t full[4], empty[4], done, drained;
+    __shared__ uint32_t tmem_base;
+    __shared__ int failed;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int co0 = blockIdx.y * CO;
+    if (tid == 0) {
+        for (int i = 0; i < 4; ++i) {
+            tc::mbar_init(tc::smem_u32(&full[i]), kLoaders / 32);
+            tc::mbar_init(tc::smem_u32(&empty[i]), 1);
+        }
+        tc::mbar_init(tc::smem_u32(&done), 1);
+        tc::mbar_init(tc::smem_u32(&drained), 128);
+        failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc::smem_u32(&tmem_base)),
+                     "r"(pl.cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    // weights: order o (input line y = o modulo 3), chunk, dx, K half, row (dz = +1, 0, -1) x slot x CO, 8 channels.
+    // Slot s of order o holds the output line yo = s modulo 3 among o - 1, o, o + 1: tap dy = y - yo.
+    for (int i = tid; i < WBYTES / 16; i += 256) {
+        const int row = i % (9 * CO), q = i / (9 * CO);
+        const int h = q & 1, blk = q >> 1;
+        const int dx = blk % 3, c = blk / 3 % NCH, o = blk / (3 * NCH);
+        const int zb = row / (3 * CO), s = row / CO % 3;
+        const int dy = (o - s + 4) % 3 - 1;   // (o - s) modulo 3 in -1, 0, 1
+        const int tap = (2 - zb) * 9 + (dy + 1) * 3 + dx;
+        *reinterpret_cast<uint4 *>(smem + (size_t)i * 16) = __ldg(reinterpret_cast<const uint4 *>(
+            w + ((int64_t)tap * COUT + co0 + row % CO) * CIN + c * 16 + h * 8));
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = tmem_base;
+    const uint32_t wbase = tc::smem_u32(smem), ring = wbase + WBYTES;
+    const int mine = (int)blockIdx.x < pl.tiles ? (pl.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+
+    struct Block {
+        int x0, y0, z0, b, ny;   // ny output lines
+    };
+    auto block_at = [&](int k) {
+        int tile = (int)blockIdx.x + k * (int)gridDim.x;
+        Block q;
+        q.x0 = tile % pl.ntx * pl.TX;
+        tile /= pl.ntx;
+        q.z0 = tile % pl.ntz * pl.TZ;
+        tile /= pl.ntz;
+        q.y0 = tile % pl.nys * pl.YS;
+        q.b = tile / pl.nys;
+        q.ny = min(pl.YS, pl.Y - q.y0);
+        return q;
+    };
+    auto fail = [&] {
+        atomicExch(&g_unet_error, 1);
+        *(volatile int *)&failed = 1;
+    };
+
+    if (warp >= 1 && warp <= 3) {
+        const int j = tid - 32;
+        const int lag = pl.ring > 2 ? 2 : 1;
+        const int items = 2 * pl.P * (pl.TZ + 2);
+        const uint32_t bar0 = tc::smem_u32(&full[0]);
+        auto hand_over = [&](int it) {
+            // (cp.async writes through the generic proxy, the tensor core reads through the async one)
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar0 + 8u * (it % pl.ring)) : "memory");
+        };
+        int it = 0;
+        bool ok = true;
+        for (int k = 0; k < mine && ok; ++k) {
+            const Block q = block_at(k);
+            for (int st = 0; st < (q.ny + 2) * NCH; ++st, ++it) {
+                const int slot = it % pl.ring, use = it / pl.ring;
+                if (use > 0) ok = tc::mbar_wait(tc::smem_u32(&empty[slot]), (uint32_t)(use - 1) & 1u);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    break;
+                }
+                const int line = st / NCH, c = st - line * NCH, y = q.y0 + line - 1;
+                const bool yin = y >= 0 && y < pl.Y;
+                const uint32_t dst0 = ring + slot * pl.stage;
+                const __nv_bfloat16 *row = in + (((int64_t)q.b * pl.Z) * pl.Y + (yin ? y : 0)) * pl.X * CIN + c * 16;
+                const int64_t zstep = (int64_t)pl.Y * pl.X * CIN;
+                int zr = 0, x = j >> 1;
+                const int h = j & 1;
+                for (int i = j; i < items; i += kLoaders, x += kLoaders / 2) {
+                    while (x >= pl.P) {
+                        x -= pl.P;
+                        ++zr;
+                    }
+                    const int gx = q.x0 + x - 1, gz = q.z0 + zr - 1;
+                    const bool inside = yin && gx >= 0 && gx < pl.X && gz >= 0 && gz < pl.Z;
+                    const __nv_bfloat16 *src = inside ? row + gz * zstep + (int64_t)gx * CIN + h * 8 : in;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst0 + h * pl.plane + (i >> 1) * 16),
+                                 "l"(src), "r"(inside ? 16 : 0)
+                                 : "memory");
+                }
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+                if (it >= lag) {
+                    if (lag == 2)
+                        asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+                    else
+                        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+                    hand_over(it - lag);
+                }
+            }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        if (ok)
+            for (int i = it > lag ? it - lag : 0; i < it; ++i) hand_over(i);
+        else if (lane == 0)
+            fail();
+    } else if (warp == 0) {
+        const uint32_t t0 = __shfl_sync(0xffffffffu, tmem, 0), on = lane == 0;
+        constexpr uint32_t kHi = (128u >> 4) | (1u << 14);
+        const uint32_t a_base = ((ring >> 4) & 0x3FFF) | (uint32_t)(pl.plane >> 4) << 16;
+        const uint32_t b_base = ((wbase >> 4) & 0x3FFF) | (uint32_t)(9 * CO) << 16;
+        int it = 0, step = 0;   // stages; input lines (the epilogue clears the accumulators before the first)
+        bool ok = true;
+        for (int k = 0; k < mine && ok; ++k) {
+            const Block q = block_at(k);
+            for (int line = 0; line < q.ny + 2 && ok; ++line, ++step) {
+                ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&drained), (uint32_t)step & 1u));
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const int order = (q.y0 + line - 1 + 3) % 3;
+                for (int c = 0; c < NCH && ok; ++c, ++it) {
+                    const int slot = it % pl.ring;
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait(tc::smem_u32(&full[slot]), (uint32_t)(it / pl.ring) & 1u));
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    const uint32_t a0 = a_base + (uint32_t)(slot * (pl.stage >> 4));
+                    const uint32_t b0 = b_base + (uint32_t)((order * NCH + c) * 3 * (WBLOCK / 16));
+                    for (int zr = 0; zr < pl.TZ + 2; ++zr) {   // input plane z0 + zr - 1
+                        const int lo = max(zr - 2, 0), hi = min(zr, pl.TZ - 1);
+                        const uint32_t d = t0 + (uint32_t)(lo * 3 * CO), a = a0 + (uint32_t)(zr * pl.P);
+                        const uint32_t b = b0 + (uint32_t)((lo - (zr - 2)) * 3 * CO);
+                        const uint32_t idesc = tc::instr_desc((hi - lo + 1) * 3 * CO);
+#pragma unroll
+                        for (int dx = 0; dx < 3; ++dx)
+                            tc::mma_lo(d, a + dx, b + dx * (WBLOCK / 16), kHi, idesc, 1u, on);
+                    }
+                    if (on) tc::mma_commit(tc::smem_u32(&empty[slot]));
+                }
+                // (on failure too: whoever waits for it is let go once the instructions in flight have ended)
+                if (on) {
+                    if (!ok) fail();
+                    tc::mma_commit(tc::smem_u32(&done));
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp >= 4) {
+        const int quarter = warp & 3;   // the tensor-memory lanes this warp can read
+        const uint32_t tq = tmem + ((uint32_t)(quarter * 32) << 16);
+        auto clear = [&](uint32_t col) {
+            asm volatile(
+                "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(
+                    tq + col),
+                "r"(0u)
+                : "memory");
+        };
+        auto hand_back = [&] {
+            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_u32(&drained)) : "memory");
+        };
+        float bv[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) bv[i] = bias ? __ldg(bias + co0 + i) : 0.f;
+        int step = 0;
+        bool ok = true;
+        for (int k = 0; k < mine && ok; ++k) {
+            const Block q = block_at(k);
+            const int pos = quarter * 32 + lane, x = q.x0 + pos;
+            const bool xin = pos < pl.TX && x < pl.X;
+            // before a block every accumulator is cleared
+            for (int col = 0; col < pl.TZ * 3; ++col) clear((uint32_t)(col * CO));
+            hand_back();
+            for (int line = 0; line < q.ny + 2; ++line, ++step) {
+                ok = tc::mbar_wait(tc::smem_u32(&done), (uint32_t)step & 1u) && !*(volatile int *)&failed;
+                if (!__all_sync(0xffffffffu, ok)) {
+                    ok = false;
+                    if (lane == 0) fail();
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                // the input line y is in: the output line y - 1 is complete
+                const int yo = q.y0 + line - 2, slot = (yo + 3) % 3;
+                for (int zo = 0; zo < pl.TZ; ++zo) {
+                    const uint32_t col = (uint32_t)((zo * 3 + slot) * CO);
+                    if (line >= 2 && q.z0 + zo < pl.Z) {
+                        float acc[16];
+                        __syncwarp();
+                        tc::tmem_ld16(tq + col, acc);
+                        if (xin) {
+                            const int64_t vo = (((int64_t)q.b * pl.Z + q.z0 + zo) * pl.Y + yo) * pl.X + x;
+                            __nv_bfloat16 m16[16];
+                            if (MASK) {
+                                const uint4 *mp = reinterpret_cast<const uint4 *>(mask + vo * COUT + co0);
+                                *reinterpret_cast<uint4 *>(m16) = __ldg(mp);
+                                *reinterpret_cast<uint4 *>(m16 + 8) = __ldg(mp + 1);
+                            }
+                            uint32_t packed[8];
+#pragma unroll
+                            for (int i = 0; i < 16; i += 2) {
+                                float lo = acc[i] + bv[i], hi = acc[i + 1] + bv[i + 1];
+                                if (RELU) {
+                                    lo = fmaxf(lo, 0.f);
+                                    hi = fmaxf(hi, 0.f);
+                                }
+                                if (MASK) {
+                                    if (!(__bfloat162float(m16[i]) > 0.f)) lo = 0.f;
+                                    if (!(__bfloat162float(m16[i + 1]) > 0.f)) hi = 0.f;
+                                }
+                                const __nv_bfloat162 pr = __floats2bfloat162_rn(lo, hi);
+                                packed[i / 2] = *reinterpret_cast<const uint32_t *>(&pr);
+                            }
+                            uint4 *op = reinterpret_cast<uint4 *>(out + vo * COUT + co0);
+                            op[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                            op[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                        }
+                    }
+                    __syncwarp();
+                    clear(col);
+                }
+                // the next line's instructions add to every slot; after a block's last line the clearing
+                // at the start of the next one hands the accumulators back
+                if (line + 1 < q.ny + 2) hand_back();
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(pl.cols) : "memory");
+    }
+}
+
 #define OMB_TC_SHAPES(X) X(16, 16) X(16, 32) X(32, 32) X(32, 64) X(64, 64) X(96, 32) X(48, 16) \
     X(32, 16) X(64, 32) X(32, 96) X(16, 48)
 
@@ -457,9 +740,90 @@ static int conv_launch(const ConvPlan &pl, const __nv_bfloat16 *in, const __nv_b
     return OMB_OK;
 }
 
+// Block shape of k_conv3d_lines: the least estimated tensor-core time over what
+// fits (three instructions of 128 clocks per input line and chunk, an epilogue of
+// about 250 clocks per output line that only a second CTA on the SM hides).
+static LinePlan line_plan(int cin, int groups, int X, int Y, int Z, int B) {
+    LinePlan best{};
+    double best_cost = 1e300;
+    const int nch = cin / 16, wbytes = 3 * nch * 3 * 9 * 16 * 32;
+    for (int occ = 2; occ >= 1; --occ)
+        for (int tz = 1; tz <= 10 && (tz <= Z || tz == 1); ++tz) {
+            LinePlan p{X, Y, Z, B};
+            p.ntx = (X + 127) / 128;
+            p.TX = (X + p.ntx - 1) / p.ntx;
+            p.TZ = tz;
+            p.P = p.TX + 2;
+            p.occ = occ;
+            if (tz * 48 > (occ == 2 ? 256 : 512)) continue;
+            for (p.cols = 32; p.cols < tz * 48;) p.cols *= 2;
+            p.plane = ((tz + 2) * p.P * 16 + 127) / 128 * 128;
+            p.stage = 2 * p.plane;
+            const int pad = 128 * 16;   // the last line's M = 128 rows read past it
+            for (p.ring = 4; p.ring >= 2 && wbytes + p.ring * p.stage + pad > (occ == 2 ? kHalfSmem : 226 * 1024);) --p.ring;
+            if (p.ring < 2) continue;
+            p.smem = wbytes + p.ring * p.stage + pad;
+            p.ntz = (Z + tz - 1) / tz;
+            const int slots = num_sms() * occ / groups;
+            const int64_t columns = (int64_t)p.ntx * p.ntz * B;
+            for (int nys = 1; nys <= Y && nys <= 64; ++nys) {
+                p.YS = (Y + nys - 1) / nys;
+                p.nys = (Y + p.YS - 1) / p.YS;
+                const int64_t tiles = columns * p.nys;
+                if (tiles > 0x7fffffff / 4096 || (int64_t)(p.YS + 2) * nch > 0x7fffff) continue;
+                p.tiles = (int)tiles;
+                const double mma = (double)(p.YS + 2) * nch * (tz + 2) * 3 * 128, epi = (double)(p.YS + 2) * (400 + 250 * tz);
+                const double per = occ == 2 ? (2 * mma > mma + epi ? 2 * mma : mma + epi) : mma + epi;
+                const double cost = (double)((tiles + slots - 1) / slots) * per;
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best = p;
+                }
+            }
+        }
+    return best;
+}
+
+template <int CIN, int COUT, bool RELU, bool MASK>
+static int lines_launch(const LinePlan &pl, const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias,
+                        __nv_bfloat16 *out, const __nv_bfloat16 *mask, cudaStream_t st) {
+    auto kernel = k_conv3d_lines<CIN, COUT, RELU, MASK>;
+    OMB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem));
+    const int slots = num_sms() * pl.occ / (COUT / 16);
+    const int grid = pl.tiles < slots ? pl.tiles : slots;
+    kernel<<<dim3(grid, COUT / 16), 256, pl.smem, st>>>(pl, in, w, bias, out, mask);
+    OMB_LAUNCH_CHECK("tcgen05 conv launch");
+    return OMB_OK;
+}
+
 template <int CIN, int COUT>
 static int conv_shape(const __nv_bfloat16 *in, const __nv_bfloat16 *w, const float *bias, __nv_bfloat16 *out,
                       const __nv_bfloat16 *mask, int relu, int X, int Y, int Z, int B, cudaStream_t st) {
+    // Lines that fill more than half of M, up to 48 channels on either side (the
+    // network's full-resolution layers): the kernel that marches along them.
+    // Shorter lines would leave most of M empty there, and wider layers' weights
+    // do not fit in three orders.
+    if constexpr (CIN <= 48 && COUT <= 48) {
+        const int ntx = (X + 127) / 128, tx = (X + ntx - 1) / ntx;
+        if (tx > 64) {
+            static thread_local LinePlan lines[8];
+            static thread_local int at = 0;
+            const LinePlan *lp = nullptr;
+            for (const LinePlan &p : lines)
+                if (p.tiles > 0 && p.X == X && p.Y == Y && p.Z == Z && p.B == B) lp = &p;
+            if (!lp) {
+                lines[at] = line_plan(CIN, COUT / 16, X, Y, Z, B);
+                lp = &lines[at];
+                at = (at + 1) % 8;
+            }
+            if (lp->tiles > 0) {
+                const LinePlan p = *lp;
+                if (mask) return lines_launch<CIN, COUT, false, true>(p, in, w, bias, out, mask, st);
+                if (relu) return lines_launch<CIN, COUT, true, false>(p, in, w, bias, out, mask, st);
+                return lines_launch<CIN, COUT, false, false>(p, in, w, bias, out, mask, st);
+            }
+        }
+    }
     // output channels of a CTA: all of them up to 48 (their weights and three
     // planes of accumulators must fit), else thirds or halves
     constexpr int CO = COUT <= 48 ? COUT : (COUT % 48 == 0 ? 48 : 32);
