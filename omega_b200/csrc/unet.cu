@@ -126,7 +126,10 @@ __global__ void __launch_bounds__(128) k_conv3d(const bf16 *__restrict__ in, con
 // channels and KS of them share the voxels.  Bound by the tensor cores'
 // m16n8k16 rate with the operand loads beside it; one tap per block of a 27-fold
 // grid, as it was before, staged both operands again for each tap
-// (training step at 128 x 128 x 64 x 4: 19.1 -> 11.8 ms).
+// (training step at 128 x 128 x 64 x 4: 19.1 -> 11.8 ms).  The copies and the operand
+// addresses advance without divisions or line loops: at that size 16 -> 16 channels
+// 437 to 408 us, 48 -> 16 1106 to 1063, 16 -> 48 998 to 940; eight warps to the
+// voxels of a 16 -> 16 stage instead of four 453.
 // ---------------------------------------------------------------------------
 struct WgradPlan {
     int X, Y, Z, B;
@@ -135,6 +138,7 @@ struct WgradPlan {
     int ring;              // stages in shared memory
     int in_plane, dz_plane, dz_off, stage;   // bytes
     int flush;             // stages whose sums a warp adds up before they go to dw
+    uint32_t inv;          // 65536 / (TX / 16) + 1: s * inv >> 16 is s / (TX / 16) for every group s of a stage
     int smem;
 };
 
@@ -150,7 +154,9 @@ struct WgradShape {
     static constexpr int MT = COUT / 16, NT = CIN / 8;
     static constexpr int MTW = MT <= 3 ? MT : 2, NTW = NT <= 2 ? NT : (MTW == 1 && NT == 6 ? 6 : (MTW == 3 ? 2 : 4));
     static constexpr int MS = MT / MTW, NS = NT / NTW;
+    static constexpr int kSums = 3 * MTW * NTW * 4;   // accumulators of a thread
     static constexpr int KS = MS * NS >= 4 ? 1 : 4 / (MS * NS);
+    static constexpr bool kPairs = kSums <= 72;       // (registers)
     static constexpr int kWarps = 3 * MS * NS * KS, kThreads = 32 * kWarps;
     static_assert(MT % MTW == 0 && NT % NTW == 0 && NTW % 2 == 0 && 3 * MTW * NTW * 4 <= 96, "wgrad tiles");
     static_assert(kThreads % (CIN / 8) == 0 && kThreads % (COUT / 8) == 0, "copy loops");
@@ -183,6 +189,36 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUT>::kThreads, 1)
     auto copy16 = [](uint32_t dst, const bf16 *src, bool ok) {
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
     };
+    // 16-byte rows of one operand: this thread's channels are fixed, and it goes from
+    // a row to the one `step` rows on without a division
+    struct Rows {
+        int c, x, line, dx, dl;
+    };
+    auto rows = [&](int c8, int pitch) {
+        const int step = S::kThreads / c8, x = tid / c8;
+        return Rows{tid % c8, x % pitch, x / pitch, step % pitch, step / pitch};
+    };
+    const Rows ri = rows(CI8, pl.TX), rd = rows(CO8, P);
+    auto copy_rows = [&](const Rows &r, uint32_t dst, const bf16 *src, int c8, int pitch, int lines, int x0, int y0, bool zin) {
+        // src: channels of the plane's voxel 0; x0, y0: voxel of the stage's row 0
+        const int chan = c8 * 8;
+        int x = r.x, gy = r.line + y0;
+        const bf16 *p = src + ((int64_t)gy * pl.X + x0 + x) * chan + r.c * 8;
+        const int64_t inc = ((int64_t)r.dl * pl.X + r.dx) * chan, wrap = (int64_t)(pl.X - pitch) * chan;
+        const uint32_t end = dst + (uint32_t)(lines * pitch) * 16u;
+        for (dst += (uint32_t)(tid / c8) * 16u; dst < end; dst += (uint32_t)(S::kThreads / c8) * 16u) {
+            const bool ok = zin && (unsigned)(x0 + x) < (unsigned)pl.X && (unsigned)gy < (unsigned)pl.Y;
+            copy16(dst, ok ? p : src, ok);
+            x += r.dx;
+            gy += r.dl;
+            p += inc;
+            if (x >= pitch) {
+                x -= pitch;
+                ++gy;
+                p += wrap;
+            }
+        }
+    };
     // requests stage k of this block's sequence
     auto load = [&](int k) {
         int tile = (int)blockIdx.x + k * (int)gridDim.x;
@@ -193,36 +229,10 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUT>::kThreads, 1)
         const int z = tile % pl.Z, b = tile / pl.Z, zi = z + dzi;
         const uint32_t st = base + (uint32_t)(k % pl.ring) * pl.stage;
         const bool zin = zi >= 0 && zi < pl.Z;
-        const bf16 *ip = in + ((int64_t)b * pl.Z + (zin ? zi : 0)) * pl.Y * pl.X * CIN;
-        const bf16 *dp = dz + ((int64_t)b * pl.Z + z) * pl.Y * pl.X * COUT;
-        {
-            const int c = tid % CI8;
-            int x = tid / CI8, line = 0;
-            const uint32_t dst = st + c * pl.in_plane;
-            for (int q = x; q < (pl.TY + 2) * pl.TX; q += S::kThreads / CI8, x += S::kThreads / CI8) {
-                while (x >= pl.TX) {
-                    x -= pl.TX;
-                    ++line;
-                }
-                const int gx = x0 + x, gy = y0 + line - 1;
-                const bool ok = zin && gx < pl.X && gy >= 0 && gy < pl.Y;
-                copy16(dst + q * 16, ok ? ip + ((int64_t)gy * pl.X + gx) * CIN + c * 8 : in, ok);
-            }
-        }
-        {
-            const int c = tid % CO8;
-            int x = tid / CO8, line = 0;
-            const uint32_t dst = st + pl.dz_off + c * pl.dz_plane;
-            for (int q = x; q < pl.TY * P; q += S::kThreads / CO8, x += S::kThreads / CO8) {
-                while (x >= P) {
-                    x -= P;
-                    ++line;
-                }
-                const int gx = x0 + x - 1, gy = y0 + line;
-                const bool ok = gx >= 0 && gx < pl.X && gy < pl.Y;
-                copy16(dst + q * 16, ok ? dp + ((int64_t)gy * pl.X + gx) * COUT + c * 8 : dz, ok);
-            }
-        }
+        copy_rows(ri, st + ri.c * pl.in_plane, in + ((int64_t)b * pl.Z + (zin ? zi : 0)) * pl.Y * pl.X * CIN, CI8, pl.TX,
+                  pl.TY + 2, x0, y0 - 1, zin);
+        copy_rows(rd, st + pl.dz_off + rd.c * pl.dz_plane, dz + ((int64_t)b * pl.Z + z) * pl.Y * pl.X * COUT, CO8, P, pl.TY,
+                  x0 - 1, y0, true);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
     auto flush = [&] {
@@ -265,53 +275,42 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUT>::kThreads, 1)
         // input: matrices (voxels 0-7 / 8-15) of two channel planes; dz: two planes for each half of the voxels
         const uint32_t ib = st + (ns * NTW + (mi >> 1)) * pl.in_plane + ((mi & 1) * 8 + rr) * 16;
         const uint32_t db = st + pl.dz_off + (ms * MTW * 2 + (mi & 1)) * pl.dz_plane + ((mi >> 1) * 8 + rr) * 16;
-        // two groups of 16 voxels at a time: the operands of the second are on
-        // their way while the first's are multiplied
-        int line = 0, x = ks * 16;
-        auto next = [&](uint32_t &ia, uint32_t &da) {
-            while (x >= pl.TX) {
-                x -= pl.TX;
-                ++line;
-            }
-            ia = ib + (uint32_t)((line + dy) * pl.TX + x) * 16u;
-            da = db + (uint32_t)(line * P + x) * 16u;
-            x += S::KS * 16;
+        auto fetch = [&](int s, uint32_t (&bq)[NTW / 2][4], uint32_t (&aq)[3][MTW][4]) {
+            const int line = (int)((uint32_t)s * pl.inv >> 16);   // s / (TX / 16)
+            const uint32_t ia = ib + (uint32_t)(dy * pl.TX + s * 16) * 16u, da = db + (uint32_t)(s * 16 + line * 2) * 16u;
+#pragma unroll
+            for (int n = 0; n < NTW / 2; ++n) ldmatrix_x4_trans(bq[n], ia + 2 * n * pl.in_plane);
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+#pragma unroll
+                for (int m = 0; m < MTW; ++m)
+                    // tap dx = d - 1 pairs input voxel u with dz voxel u - dx, staged at u - dx + 1
+                    ldmatrix_x4_trans(aq[d][m], da + (2 - d) * 16 + 2 * m * pl.dz_plane);
         };
-        constexpr int G = MTW * NTW * 12 <= 72 ? 2 : 1;   // (registers)
-        for (int s = ks; s < total; s += G * S::KS) {
-            const bool two = G > 1 && s + S::KS < total;
-            uint32_t ia[G], da[G], bq[G][NTW / 2][4];
-            next(ia[0], da[0]);
-            if (two) next(ia[G - 1], da[G - 1]);
+        auto multiply = [&](const uint32_t (&bq)[NTW / 2][4], const uint32_t (&aq)[3][MTW][4]) {
 #pragma unroll
-            for (int u = 0; u < G; ++u)
-                if (u == 0 || two) {
+            for (int d = 0; d < 3; ++d)
 #pragma unroll
-                    for (int n = 0; n < NTW / 2; ++n) ldmatrix_x4_trans(bq[u][n], ia[u] + 2 * n * pl.in_plane);
-                }
-            uint32_t aq[G][3][MTW][4];
+                for (int m = 0; m < MTW; ++m)
 #pragma unroll
-            for (int u = 0; u < G; ++u)
-                if (u == 0 || two) {
-#pragma unroll
-                    for (int d = 0; d < 3; ++d)
-#pragma unroll
-                        for (int m = 0; m < MTW; ++m)
-                            // tap dx = d - 1 pairs input voxel u with dz voxel u - dx, staged at u - dx + 1
-                            ldmatrix_x4_trans(aq[u][d][m], da[u] + (2 - d) * 16 + 2 * m * pl.dz_plane);
-                }
-#pragma unroll
-            for (int u = 0; u < G; ++u)
-                if (u == 0 || two) {
-#pragma unroll
-                    for (int d = 0; d < 3; ++d)
-#pragma unroll
-                        for (int m = 0; m < MTW; ++m)
-#pragma unroll
-                            for (int n = 0; n < NTW; ++n)
-                                mma_bf16(acc[d][m][n], aq[u][d][m][0], aq[u][d][m][1], aq[u][d][m][2], aq[u][d][m][3],
-                                         bq[u][n / 2][(n & 1) * 2], bq[u][n / 2][(n & 1) * 2 + 1]);
-                }
+                    for (int n = 0; n < NTW; ++n)
+                        mma_bf16(acc[d][m][n], aq[d][m][0], aq[d][m][1], aq[d][m][2], aq[d][m][3], bq[n / 2][(n & 1) * 2],
+                                 bq[n / 2][(n & 1) * 2 + 1]);
+        };
+        uint32_t bq[2][NTW / 2][4], aq[2][3][MTW][4];
+        int s = ks;
+        // two groups of 16 voxels at a time, where the registers allow: the operands of the
+        // second are on their way while the first's are multiplied
+        if constexpr (S::kPairs)
+            for (; s + S::KS < total; s += 2 * S::KS) {
+                fetch(s, bq[0], aq[0]);
+                fetch(s + S::KS, bq[1], aq[1]);
+                multiply(bq[0], aq[0]);
+                multiply(bq[1], aq[1]);
+            }
+        for (; s < total; s += S::KS) {
+            fetch(s, bq[0], aq[0]);
+            multiply(bq[0], aq[0]);
         }
         // sums of at most about 8192 voxels are added up before they go to memory
         if ((k + 1) % pl.flush == 0 && k + 1 < mine) {
@@ -844,6 +843,7 @@ static int launch_wgrad(const bf16 *in, const bf16 *dz, float *dw, int X, int Y,
         if (p.smem) break;
     }
     p.nty = (Y + p.TY - 1) / p.TY;
+    p.inv = 65536u / (p.TX / 16) + 1;   // (at most 64 groups of a stage, 8 of a line: exact)
     const int64_t tiles = (int64_t)p.ntx * p.nty * Z * B;
     if (!p.smem || tiles > 2147483647) return set_error(OMB_ERR_UNSUPPORTED, "wgrad volume too large");
     p.tiles = (int)tiles;
