@@ -128,8 +128,7 @@ __global__ void __launch_bounds__(128) k_conv3d(const bf16 *__restrict__ in, con
 // grid, as it was before, staged both operands again for each tap
 // (training step at 128 x 128 x 64 x 4: 19.1 -> 11.8 ms).  The copies and the operand
 // addresses advance without divisions or line loops: at that size 16 -> 16 channels
-// 437 to 408 us, 48 -> 16 1106 to 1063, 16 -> 48 998 to 940; eight warps to the
-// voxels of a 16 -> 16 stage instead of four 453.
+// 437 to 408 us, 48 -> 16 1106 to 1063, 16 -> 48 998 to 940.
 // ---------------------------------------------------------------------------
 struct WgradPlan {
     int X, Y, Z, B;
@@ -267,10 +266,6 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUT>::kThreads, 1)
         else
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
         __syncthreads();   // stage k is here for everybody, and everybody is done with stage k - 1
-        if (k + pl.ring - 1 < mine)
-            load(k + pl.ring - 1);
-        else
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
         const uint32_t st = base + (uint32_t)(k % pl.ring) * pl.stage;
         // input: matrices (voxels 0-7 / 8-15) of two channel planes; dz: two planes for each half of the voxels
         const uint32_t ib = st + (ns * NTW + (mi >> 1)) * pl.in_plane + ((mi & 1) * 8 + rr) * 16;
@@ -299,18 +294,35 @@ __global__ void __launch_bounds__(WgradShape<CIN, COUT>::kThreads, 1)
         };
         uint32_t bq[2][NTW / 2][4], aq[2][3][MTW][4];
         int s = ks;
-        // two groups of 16 voxels at a time, where the registers allow: the operands of the
-        // second are on their way while the first's are multiplied
-        if constexpr (S::kPairs)
-            for (; s + S::KS < total; s += 2 * S::KS) {
-                fetch(s, bq[0], aq[0]);
-                fetch(s + S::KS, bq[1], aq[1]);
-                multiply(bq[0], aq[0]);
-                multiply(bq[1], aq[1]);
+        // a third of the warps of a scheduler requests the stage after next before its groups,
+        // a third between them and a third after them, so that the copies' issue does not stop
+        // the tensor cores (with two stages they would come too late); all before their groups,
+        // at 128 x 128 x 64 x 4: 16 -> 16 channels 408 us, now 304; 48 -> 16 1063, now 759;
+        // 16 -> 48 940, now 662
+        const int phase = pl.ring == 3 ? (warp >> 2) % 3 : 0;
+#pragma unroll 1
+        for (int part = 0;; ++part) {
+            if (part == phase) {
+                if (k + pl.ring - 1 < mine)
+                    load(k + pl.ring - 1);
+                else
+                    asm volatile("cp.async.commit_group;\n" ::: "memory");
             }
-        for (; s < total; s += S::KS) {
-            fetch(s, bq[0], aq[0]);
-            multiply(bq[0], aq[0]);
+            if (part == 2) break;
+            const int stop = part == 0 ? total / 2 : total;
+            // two groups of 16 voxels at a time, where the registers allow: the operands of the
+            // second are on their way while the first's are multiplied
+            if constexpr (S::kPairs)
+                for (; s + S::KS < stop; s += 2 * S::KS) {
+                    fetch(s, bq[0], aq[0]);
+                    fetch(s + S::KS, bq[1], aq[1]);
+                    multiply(bq[0], aq[0]);
+                    multiply(bq[1], aq[1]);
+                }
+            for (; s < stop; s += S::KS) {
+                fetch(s, bq[0], aq[0]);
+                multiply(bq[0], aq[0]);
+            }
         }
         // sums of at most about 8192 voxels are added up before they go to memory
         if ((k + 1) % pl.flush == 0 && k + 1 < mine) {
