@@ -554,21 +554,35 @@ __global__ void k_avgpool2_bwd_v8(const uint4 *__restrict__ dout, uint4 *__restr
     }
 }
 
+// A block takes whole lines, so that the line's place is found once (the
+// divisions of a flat index were most of the kernel), and a thread has
+// kUpLoads reads on their way before its first write.  32 + 16 channels at
+// 128 x 128 x 64 x 4: 193 us with a flat index and one read at a time, 154 with
+// four reads, 106 so (a training step 6288 -> 6186 us).
+constexpr int kUpLoads = 4;
 __global__ void k_up_concat_v8(const uint4 *__restrict__ low, const uint4 *__restrict__ skip, uint4 *__restrict__ cat,
-                               int X, int Y, int Z, int L8, int S8, int64_t n) {
-    const int C8 = L8 + S8;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = i <= 0xffffffffll ? (unsigned)i / (unsigned)C8 : i / C8;
-        const int c = (int)(i - v * C8);
-        if (c >= L8) {
-            cat[i] = __ldg(skip + v * S8 + (c - L8));
-        } else {
-            const Vox q = voxel_at(v, X, Y, Z);
-            cat[i] = __ldg(low + vox_index(q.b, q.z / 2, q.y / 2, q.x / 2, Z / 2, Y / 2, X / 2) * L8 + c);
+                               int X, int Y, int Z, int L8, int S8, int64_t lines) {
+    const unsigned C8 = L8 + S8, row = X * C8;
+    for (int64_t l = blockIdx.x; l < lines; l += gridDim.x) {
+        const int y = (int)(l % Y), z = (int)(l / Y % Z);
+        const int64_t b = l / Y / Z;
+        const uint4 *lp = low + vox_index(b, z / 2, y / 2, 0, Z / 2, Y / 2, X / 2) * L8, *sp = skip + l * X * S8;
+        uint4 *op = cat + l * row;
+        for (unsigned e0 = threadIdx.x; e0 < row; e0 += kUpLoads * blockDim.x) {
+            uint4 r[kUpLoads];
+#pragma unroll
+            for (int u = 0; u < kUpLoads; ++u) {
+                const unsigned e = e0 + u * blockDim.x;
+                if (e >= row) continue;
+                const unsigned x = e / C8, c = e - x * C8;
+                r[u] = __ldg(c < (unsigned)L8 ? lp + (x / 2) * L8 + c : sp + x * S8 + (c - L8));
+            }
+#pragma unroll
+            for (int u = 0; u < kUpLoads; ++u)
+                if (e0 + u * blockDim.x < row) op[e0 + u * blockDim.x] = r[u];
         }
     }
 }
-
 __global__ void k_up_concat_bwd_v8(const uint4 *__restrict__ dcat, uint4 *__restrict__ dlow, uint4 *__restrict__ dskip,
                                    int X, int Y, int Z, int L8, int S8, int64_t n_low, int64_t n) {
     const int C8 = L8 + S8;
@@ -930,11 +944,12 @@ int unet_avgpool(const void *in, void *out, int X, int Y, int Z, int B, int C, i
 
 int unet_up_concat(const void *low, const void *skip, void *cat, int X, int Y, int Z, int B, int cl, int cs,
                    cudaStream_t st) {
-    const int64_t nvox = (int64_t)X * Y * Z * B;
-    if (vec8({low, skip, cat}, cl) && cs % 8 == 0) {
-        const int64_t n = nvox * ((cl + cs) / 8);
-        k_up_concat_v8<<<grid_for(n, 8), 256, 0, st>>>(static_cast<const uint4 *>(low), static_cast<const uint4 *>(skip),
-                                                       static_cast<uint4 *>(cat), X, Y, Z, cl / 8, cs / 8, n);
+    const int64_t nvox = (int64_t)X * Y * Z * B, lines = (int64_t)Y * Z * B;
+    // (a line's 16-byte words are counted in 32 bits)
+    if (vec8({low, skip, cat}, cl) && cs % 8 == 0 && X > 0 && lines > 0 && (int64_t)X * ((cl + cs) / 8) < 0x40000000) {
+        k_up_concat_v8<<<grid_for(lines, 8, 1), 256, 0, st>>>(static_cast<const uint4 *>(low),
+                                                              static_cast<const uint4 *>(skip), static_cast<uint4 *>(cat),
+                                                              X, Y, Z, cl / 8, cs / 8, lines);
         OMB_LAUNCH_CHECK("upsample launch");
         return OMB_OK;
     }
