@@ -279,7 +279,8 @@ typedef struct omb_tuning {
                                         loads are in flight per thread */
     int32_t bdd_fp_staged;           /* 0, 1 (default 1): type-5 forward projection with each CTA's
                                         per-slice image boxes staged in shared memory by TMA (applies
-                                        with bdd_fp_columns = 8; needs Nx, Ny multiples of 4) */
+                                        with bdd_fp_columns = 8 or 16; needs Nx, Ny multiples of
+                                        4) */
     int32_t bdd_bp_staged;           /* 0, 1 (default 1): type-5 backprojection with each CTA's
                                         per-projection detector boxes staged in shared memory by TMA
                                         (applies with bdd_bp_zrun = 8 or 16; needs a row count that is a
