@@ -54,22 +54,22 @@ PROFILED_TRAFFIC = {
     # DRAM bytes read + written per launch, from the ncu captures summarised
     # in profiles/: bdd_cbct_capture.md (36-view capture x 10) and
     # siddon_dynpet_launches.md (full-size capture)
-    ("cbct", "bdd_fp"): 9.46e9,
-    ("cbct", "bdd_bp"): 3.76e8,
+    ("cbct", "bdd_fp"): 1.095e10,
+    ("cbct", "bdd_bp"): 3.93e8,
     ("dynpet", "siddon_fp"): 3.81e8,
     ("dynpet", "siddon_bp"): 6.59e9,   # 3 launches of k_sm_bp_sl (8 frames each) per call
     # interp_tof_capture.md: one subset's forward launch (16 per step)
-    ("interp_tof", "interp_fp"): 5.60e6,
+    ("interp_tof", "interp_fp"): 6.61e6,
 }
 # What bounds each kernel instead of HBM (the volumes and images are
 # L2-resident, so DRAM moves a few per cent of the cache-less bytes): the
 # issue-active and SM-throughput percentages of the same ncu captures.
 PROFILED_LIMITER = {
-    ("cbct", "bdd_fp"): {"issue_active_pct": 80.4, "sm_throughput_pct": 75.5, "dram_pct": 7.6},
-    ("cbct", "bdd_bp"): {"issue_active_pct": 72.9, "sm_throughput_pct": 71.8, "dram_pct": 0.35},
+    ("cbct", "bdd_fp"): {"issue_active_pct": 72.9, "sm_throughput_pct": 65.2, "dram_pct": 11.5},
+    ("cbct", "bdd_bp"): {"issue_active_pct": 75.8, "sm_throughput_pct": 74.8, "dram_pct": 0.40},
     ("dynpet", "siddon_fp"): {"issue_active_pct": 66.5, "l1tex_pct": 92.0, "dram_pct": 1.0},
     ("dynpet", "siddon_bp"): {"issue_active_pct": 10.7, "l1tex_pct": 94.0, "dram_pct": 21.8},
-    ("interp_tof", "interp_fp"): {"issue_active_pct": 84.9, "sm_throughput_pct": 78.6, "dram_pct": 0.01},
+    ("interp_tof", "interp_fp"): {"issue_active_pct": 72.3, "sm_throughput_pct": 64.8, "dram_pct": 0.06},
 }
 FALLBACK_HBM_GBS = 6650.0
 
