@@ -623,21 +623,38 @@ __global__ void k_relu_mask_v8(uint4 *__restrict__ d, const uint4 *__restrict__ 
     }
 }
 
-// Bias gradient, 8 channels per thread: C8 threads side by side take a voxel.
-__global__ void __launch_bounds__(256) k_bias_grad_v8(const uint4 *__restrict__ dz, float *__restrict__ db, int C8,
-                                                      int64_t n) {
-    __shared__ float part[256][9];
+// Bias gradient, 8 channels per thread: C8 (2, 4 or 8) threads side by side take
+// a voxel.  Few large blocks and a tree inside each, because the FP32 additions
+// of the blocks' sums are what the rounding of the result comes from.  4.2M x 16,
+// 524288 x 32 and 65536 x 64 values: relative error 1.9e-7, 2.0e-7 and 1.4e-7;
+// with 592 blocks of 256 threads 3.7e-7, 5.0e-7 and 2.6e-7 (a training step's ten
+// launches 174 us, were 151).
+constexpr int kBiasThreads = 1024, kBiasLoads = 4;
+__global__ void __launch_bounds__(kBiasThreads) k_bias_grad_v8(const uint4 *__restrict__ dz, float *__restrict__ db, int C8,
+                                                               int64_t n) {
+    __shared__ float part[kBiasThreads / 32][64];
     float s[8] = {};
-    const int64_t stride = (int64_t)gridDim.x * 256;   // (a multiple of C8: a thread keeps its channels)
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += stride) add8(s, __ldg(dz + i));
+    const int64_t stride = (int64_t)gridDim.x * kBiasThreads;   // (a multiple of C8: a thread keeps its channels)
+    for (int64_t i = (int64_t)blockIdx.x * kBiasThreads + threadIdx.x; i < n; i += kBiasLoads * stride) {
+        uint4 q[kBiasLoads];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) part[threadIdx.x][k] = s[k];
+        for (int u = 0; u < kBiasLoads; ++u) q[u] = i + u * stride < n ? __ldg(dz + i + u * stride) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < kBiasLoads; ++u) add8(s, q[u]);
+    }
+    const int lane = threadIdx.x & 31;
+    for (int o = 16; o >= C8; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+    if (lane < C8)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) part[threadIdx.x >> 5][lane * 8 + k] = s[k];
     __syncthreads();
-    const int c = threadIdx.x;
-    if (c < 8 * C8) {
-        float t = 0.f;
-        for (int r = c / 8; r < 256; r += C8) t += part[r][c & 7];
-        atomicAdd(db + c, t);
+    const int c = threadIdx.x >> 5;   // warp c adds up channels c and c + 32
+    for (int ch = c; ch < 8 * C8; ch += 32) {
+        float t = part[lane][ch];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) atomicAdd(db + ch, t);
     }
 }
 
@@ -897,7 +914,7 @@ int unet_bias_grad(int c, const void *dz, float *db, int64_t nvox, cudaStream_t 
     const bf16 *d = static_cast<const bf16 *>(dz);
     if ((c == 16 || c == 32 || c == 64) && vec8({dz}, c)) {
         const int64_t n = nvox * (c / 8);
-        k_bias_grad_v8<<<grid_for(n, 4), 256, 0, st>>>(static_cast<const uint4 *>(dz), db, c / 8, n);
+        k_bias_grad_v8<<<grid_for(n, 1, kBiasThreads), kBiasThreads, 0, st>>>(static_cast<const uint4 *>(dz), db, c / 8, n);
         OMB_LAUNCH_CHECK("bias gradient launch");
         return OMB_OK;
     }
