@@ -35,6 +35,7 @@
 //    FP64-built projective map as the type-5 backprojection instead of the
 //    FP32 plane intersection (identical in exact arithmetic).
 #include "kernels.h"
+#include "march_range.cuh"
 #include "scratch.cuh"
 #include "siddon.cuh"
 
@@ -137,20 +138,6 @@ __device__ __forceinline__ float trilinear_inside(const T *__restrict__ img, int
     const float c01 = fmaf(ax, v101 - v001, v001), c11 = fmaf(ax, v111 - v011, v011);
     const float c0 = fmaf(ay, c10 - c00, c00), c1 = fmaf(ay, c11 - c01, c01);
     return fmaf(az, c1 - c0, c0);
-}
-
-// Samples [lo, hi] of a march that lie inside on one axis (c + n s in [0, size
-// - 1), with a margin far above the rounding of c + n s); intersected into lo, hi.
-__device__ __forceinline__ void inside_range(float c, float s, int size, float &lo, float &hi) {
-    const float a = 0.01f - c, b = (float)(size - 1) - 0.01f - c;
-    if (fabsf(s) < 1e-6f) {
-        // (a sample count times 1e-6 stays far inside one voxel)
-        if (!(a <= -0.5f && b >= 0.5f)) hi = -1.f;
-        return;
-    }
-    const float p = a / s, q = b / s;
-    lo = fmaxf(lo, ceilf(fminf(p, q)));
-    hi = fminf(hi, floorf(fmaxf(p, q)));
 }
 
 // W: bins a thread keeps of a TOF measurement (tof.cuh), 0 without TOF.
