@@ -616,6 +616,10 @@ __global__ void __launch_bounds__(256) k_conv3d_lines(const __grid_constant__ Li
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 // the input line y is in: the output line y - 1 is complete
                 const int yo = q.y0 + line - 2, slot = (yo + 3) % 3;
+                // After a block's last line nothing is cleared here: the next block begins by clearing every
+                // accumulator, and after the last block the tensor memory is given back, by when every store
+                // to it has been waited for (hand_back does, so no clearing goes without one).
+                const bool more = line + 1 < q.ny + 2;
                 for (int zo = 0; zo < pl.TZ; ++zo) {
                     const uint32_t col = (uint32_t)((zo * 3 + slot) * CO);
                     if (line >= 2 && q.z0 + zo < pl.Z) {
@@ -651,11 +655,10 @@ __global__ void __launch_bounds__(256) k_conv3d_lines(const __grid_constant__ Li
                         }
                     }
                     __syncwarp();
-                    clear(col);
+                    if (more) clear(col);
                 }
-                // the next line's instructions add to every slot; after a block's last line the clearing
-                // at the start of the next one hands the accumulators back
-                if (line + 1 < q.ny + 2) hand_back();
+                // the next line's instructions add to every slot
+                if (more) hand_back();
             }
         }
     }
