@@ -43,3 +43,26 @@ def test_windowed_tof_matches_oracle(cuda, projector, bins, fwhm):
     ref, ref_s = bwd(g, m, 1, sens=True)
     assert orc.rel_l2(img.cpu().numpy(), ref) < TOL
     assert orc.rel_l2(sens.cpu().numpy(), ref_s) < TOL
+
+
+@pytest.mark.parametrize("spacing", [200.0, 900.0])
+def test_bins_far_from_the_image(cuda, spacing):
+    """Bins out to 1.4 m beside a 180 mm image (sigma 3.3 mm, elements of up to
+    4.1 mm: the series form) and out to 6.3 m.  The int64 backprojection keeps
+    all of them, and what one adds far from its centre is 0, not 0 times
+    infinity."""
+    import torch
+    from configs import CONFIGS, apply
+    from omega_b200.projector import proj
+    o = apply(proj.projectorClass(),
+              dict(CONFIGS["pet_mini"], TOF_bins=15, TOF_bins_used=15, TOF_width=spacing / (C / 2.),
+                   TOF_FWHM=3.3 * np.sqrt(8 * np.log(2.0)) * 2 / C, use_64bit_atomics=True, Nx=64, Ny=64, Nz=31))
+    o.addProjector()
+    o.initProj()
+    g = orc.Geometry(o)
+    rng = np.random.default_rng(5)
+    m = rng.poisson(2.0, g.rays(1) * g.nbins).astype(np.float32)
+    img, sens = o.backwardProject(torch.from_numpy(m).to(cuda), 1, sens=True)
+    ref, ref_s = orc.backward(g, m, 1, sens=True)
+    assert orc.rel_l2(img.cpu().numpy(), ref) < TOL
+    assert orc.rel_l2(sens.cpu().numpy(), ref_s) < TOL
