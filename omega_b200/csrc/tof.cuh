@@ -2,14 +2,15 @@
 // window of bins.
 //
 // A ray advances monotonically through the TOF bins, and a bin's Gaussian is
-// nothing next to the element's total once its centre is 8 sigma away
-// (exp(-32) against a total of at least exp(-(bin spacing / 2 sigma)^2 / 2),
-// under 2^-40).  So a thread keeps W neighbouring bins in registers, in the
+// nothing next to the element's total once its centre is much farther away than
+// the nearest one's.  So a thread keeps W neighbouring bins in registers, in the
 // order the ray meets them, instead of all of them: when the next bin outside
 // the window comes nearer than the first one inside, the first is written out
 // (forward) or dropped (backward) and the window moves on.  The host picks the
-// smallest built W whose half span covers 8 sigma plus half an element
-// (tof_setup); with closely spaced bins that is every bin and nothing slides.
+// smallest built W that leaves out only bins 8 sigma away whose weight is below
+// 2^-30 of the element's total (tof_setup); with closely spaced bins that is
+// every bin and nothing slides.  (An infinity or NaN in a measurement or voxel
+// reaches the bins of the window, not all.)
 //
 // The weight of a bin is the 4-point trapezoid of its Gaussian over the
 // element (TOFLoop / TOFWeight, general_opencl_functions.h:1077-1117).  About
@@ -197,10 +198,23 @@ inline void tof_setup(Tof &t, const float *centers, float *sorted, int *order, f
             }
     for (int i = 0; i < n; ++i) sorted[i] = centers[order[i]];
     if (!finite) return;
+    // The window moves on halfway between bins i and i + w.  There the bin left
+    // out (or not yet met) weighs most against the element's total: farther on it
+    // loses more than the nearest bin does.  The total is at least a third (the
+    // trapezoid's inner points) of the nearest bin's Gaussian a sixth of an
+    // element farther away.  Evenly spaced bins have one halfway and pass the
+    // second test with the first; bins in pairs far apart need not.
     for (int w = 2; w < n; w += 2) {
-        double half = 1e30;
-        for (int i = 0; i + w < n; ++i) half = fmin(half, 0.5 * ((double)sorted[i + w] - sorted[i]));
-        if (half >= 8.0 * sigma + 0.5 * element) {
+        bool covers = true;
+        for (int i = 0; i + w < n; ++i) {
+            const double at = 0.5 * ((double)sorted[i] + sorted[i + w]), half = at - sorted[i];
+            double nearest = half;
+            for (int j = i + 1; j < i + w; ++j) nearest = fmin(nearest, fabs(at - sorted[j]));
+            const double away = half - 0.5 * element, near = nearest + element / 6.0;
+            // 3 exp(-x / 2 sigma^2) < 2^-30 from x = 43.8 sigma^2
+            covers = covers && away >= 8.0 * sigma && away * away - near * near >= 44.0 * sigma * sigma;
+        }
+        if (covers) {
             t.window = w;
             return;
         }
