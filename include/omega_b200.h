@@ -24,6 +24,12 @@
  *  - A handle binds one device (the current device at omb_create) and is not
  *    reentrant: do not call into one handle from two threads at once.
  *    Distinct handles are independent.
+ *  - Projections of one image without TOF by types 1 and 4 take an image-sized
+ *    scratch copy from a stream-ordered pool of the device, which keeps up to
+ *    512 MB between calls and returns it with the device's last handle.  Without
+ *    the memory, and while `stream` is being captured into a CUDA graph, they
+ *    do without the copy: the same sums, up to 15 per cent slower, and no memory
+ *    nodes in the graph.
  */
 #ifndef OMEGA_B200_H
 #define OMEGA_B200_H

@@ -41,6 +41,12 @@ void scratch_drop(int device) {
 StreamScratch::StreamScratch(size_t bytes, cudaStream_t st) : stream(st) {
     int device = 0;
     if (bytes == 0) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return;
     if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= kMaxDevices) return;
     cudaMemPool_t pool;
     {

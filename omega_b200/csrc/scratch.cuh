@@ -1,9 +1,10 @@
 // Scratch memory of one call, allocated and freed in stream order, so calls on
-// several streams and threads (and captured graphs, where the pair becomes
-// graph nodes) never share it.  It comes from one pool per device that exists
-// while the device has handles: omb_create / omb_destroy hold it, the last
-// handle's end returns its memory; what it keeps between calls is bounded by
-// kScratchKept.
+// several streams and threads never share it.  It comes from one pool per device
+// that exists while the device has handles: omb_create / omb_destroy hold it,
+// the last handle's end returns its memory; what it keeps between calls is
+// bounded by kScratchKept.  A call that is being captured into a CUDA graph gets
+// none: the pair would become memory nodes, and a graph with those can be
+// neither cloned nor instantiated twice.
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -17,7 +18,7 @@ void scratch_drop(int device);
 
 struct StreamScratch {
     void *p = nullptr;
-    // p is NULL when there is no pool, no memory or bytes is 0: the caller does without
+    // p is NULL when there is no pool or memory, the stream is capturing or bytes is 0: the caller does without
     StreamScratch(size_t bytes, cudaStream_t st);
     ~StreamScratch();
     StreamScratch(const StreamScratch &) = delete;

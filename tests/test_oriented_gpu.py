@@ -49,8 +49,8 @@ def test_oriented_projections_match_oracle(cuda, projector, shape, extra):
 
 
 def test_oriented_projections_in_a_graph(cuda):
-    """The copy's memory is taken inside the call: a captured call replays with
-    the same result, also after eager calls of other images."""
+    """A captured call (which takes no copy) replays with the eager call's
+    result, also after eager calls of other images."""
     import torch
     o = _options(Nx=33, Ny=45, FOVa_x=170., FOVa_y=150.)
     n = int(o.N[0])
@@ -71,3 +71,50 @@ def test_oriented_projections_in_a_graph(cuda):
         graph.replay()
         assert torch.equal(y, want)
     del graph
+
+
+@pytest.mark.parametrize("projector", [1, 4])
+def test_captured_projections_hold_no_memory_nodes(cuda, projector):
+    """A graph with memory allocation nodes can be neither cloned nor
+    instantiated twice at once; these can, and both instances compute the
+    projections."""
+    import ctypes
+
+    import torch
+    rt = ctypes.CDLL("libcudart.so.12")
+    o = _options(Nx=33, Ny=45, FOVa_x=170., FOVa_y=150., projector_type=projector)
+    gen = torch.Generator(device=cuda).manual_seed(2)
+    x = torch.rand(int(o.N[0]), generator=gen, device=cuda)
+    want_y = o.forwardProject(x, 0).clone()
+    want_b = o.backwardProject(want_y, 0).clone()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        y = o.forwardProject(x, 0)
+        b = o.backwardProject(y, 0)
+    raw = ctypes.c_void_p(graph.raw_cuda_graph())
+    n = ctypes.c_size_t(0)
+    assert rt.cudaGraphGetNodes(raw, None, ctypes.byref(n)) == 0
+    nodes = (ctypes.c_void_p * n.value)()
+    assert rt.cudaGraphGetNodes(raw, nodes, ctypes.byref(n)) == 0
+    for node in nodes:
+        kind = ctypes.c_int(-1)
+        assert rt.cudaGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        assert kind.value not in (10, 11)   # memory allocation, memory free
+    clone = ctypes.c_void_p()
+    assert rt.cudaGraphClone(ctypes.byref(clone), raw) == 0
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    execs = []
+    for g in (raw, clone):
+        e = ctypes.c_void_p()
+        assert rt.cudaGraphInstantiate(ctypes.byref(e), g, ctypes.c_ulonglong(0)) == 0
+        execs.append(e)
+    for e in execs:
+        y.zero_()
+        b.zero_()
+        assert rt.cudaGraphLaunch(e, stream) == 0
+        torch.cuda.synchronize()
+        assert float((y - want_y).norm() / want_y.norm()) < 1e-6
+        assert float((b - want_b).norm() / want_b.norm()) < 1e-6
+    for e in execs:
+        assert rt.cudaGraphExecDestroy(e) == 0
+    assert rt.cudaGraphDestroy(clone) == 0
