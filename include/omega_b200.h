@@ -269,8 +269,14 @@ typedef struct omb_tuning {
     uint32_t struct_size;            /* sizeof(omb_tuning) */
     int32_t siddon_blocks_per_sm;    /* 1..32 (default 8): grid of the grid-stride Siddon kernels */
     int32_t siddon_frames_per_walk;  /* 1, 2, 4, 8 (default 8): most frames sharing one ray walk */
-    int32_t bdd_fp_columns;          /* 8, 16 (default 16 where the staged kernel fills the GPU with it, else 8): type-5 forward, detector columns per thread */
-    int32_t bdd_bp_zrun;             /* 4, 8, 16 (default 16 where the staged kernel fills the GPU with it, else 8): type-5 backward, voxels along z per thread */
+    int32_t bdd_fp_columns;          /* 8, 16: type-5 forward, detector columns per thread.  Default 16 where
+                                        the staged kernel fills the GPU with it, else 8.  With
+                                        bdd_fp_staged = 0 the unstaged kernel runs the value set here
+                                        (8 is the better one); with bdd_fp_staged = 1 and sizes that can
+                                        be staged, a call whose image is off a 16-byte boundary runs 8 */
+    int32_t bdd_bp_zrun;             /* 4, 8, 16: type-5 backward, voxels along z per thread.  Default 16
+                                        where the staged kernel fills the GPU with it, else 8; unstaged
+                                        calls as for bdd_fp_columns */
     int32_t bdd_fp_block_rows;       /* 4, 8 (default 8): type-5 forward, warps per block */
     int32_t bdd_bp_block_rows;       /* 4, 8 (default 8): type-5 backward, warps per block */
     int32_t siddon_frame_layout;     /* 0, 1 (default 1): type-1 non-TOF batches of >= 4 frames.

@@ -530,7 +530,8 @@ int omb_create(const omb_geometry_desc *desc, omb_handle **out) {
     // (back 3.61 -> 2.94 ms) -- where their CTAs (32 x 64 pixels of a view; 32 x 4
     // columns of voxels) still fill every SM.  The unstaged kernels spend their
     // time in memory accesses and lose with the wider threads (133 x 133 x 80,
-    // 161 x 79 x 80 views: forward, dual and back 1.78 against 2.17 ms).
+    // 161 x 79 x 80 views: forward, dual and back 1.78 against 2.17 ms); a call
+    // whose buffers cannot be staged runs 8 there (bdd_forward, bdd_backward).
     if (desc->fp_type == 5 && desc->nx % 4 == 0 && desc->ny % 4 == 0 && desc->n_cols_d >= 64 &&
         (int64_t)((desc->n_rows_d + 31) / 32) * ((desc->n_cols_d + 63) / 64) * (desc->n_proj / desc->n_subsets) >=
             6 * (int64_t)num_sms())

@@ -435,7 +435,10 @@ int bdd_forward(const Grid &g, const float *xy, const float *uv, int nr, int nc,
     if (tr != OMB_OK) return tr;
     if (tn.bdd_fp_staged && (tn.bdd_fp_cols == 8 || tn.bdd_fp_cols == 16) && bdd_fp_tma_supported(g, img, imgT))
         return bdd_forward_tma(g, xy, uv, nr, nc, pitch_y, proj0, nproj, img, imgT, y, tn.bdd_fp_cols, st);
-    switch (tn.bdd_fp_cols) {
+    // a width set for the staged kernel is not the unstaged one's: sizes that are staged, on a buffer that
+    // cannot be (off a 16-byte boundary), run 8 columns
+    const int cols = tn.bdd_fp_staged && g.nx % 4 == 0 && g.ny % 4 == 0 ? 8 : tn.bdd_fp_cols;
+    switch (cols) {
         case 16: launch_fp<16>(g, xy, uv, nr, nc, pitch_y, proj0, nproj, img, imgT, y, tn.bdd_fp_rows, st); break;
         default: launch_fp<8>(g, xy, uv, nr, nc, pitch_y, proj0, nproj, img, imgT, y, tn.bdd_fp_rows, st); break;
     }
@@ -475,7 +478,9 @@ int bdd_backward(const Grid &g, const BddProj *pj, const BddMap64 *pm, int nr, i
     if (tn.bdd_bp_staged && (tn.bdd_bp_z == 8 || tn.bdd_bp_z == 16) && bdd_bp_tma_supported(nr, y))
         return bdd_backward_tma(g, pj, pm, nr, nc, nproj, y, img, sens, tn.bdd_bp_z, st);
     const int rows = tn.bdd_bp_rows;
-    switch (tn.bdd_bp_z) {
+    // (as in the forward projection)
+    const int z = tn.bdd_bp_staged && nr % 4 == 0 && tn.bdd_bp_z == 16 ? 8 : tn.bdd_bp_z;
+    switch (z) {
         case 4: launch_bp<4>(g, pj, pm, nr, nc, nproj, y, img, sens, rows, st); break;
         case 16: launch_bp<16>(g, pj, pm, nr, nc, nproj, y, img, sens, rows, st); break;
         default: launch_bp<8>(g, pj, pm, nr, nc, nproj, y, img, sens, rows, st); break;

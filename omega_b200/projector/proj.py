@@ -1018,7 +1018,13 @@ class projectorClass:
         self._check_ready()
         t = _native.Tuning(struct_size=ctypes.sizeof(_native.Tuning))
         _native.call("omb_get_tuning", self._handle, ctypes.byref(t))
-        for k, v in dict(values).items():
+        values = dict(values)
+        # staging switched off on its own: the widths the unstaged kernels are best with
+        if t.bdd_fp_staged and not values.get("bdd_fp_staged", 1):
+            values.setdefault("bdd_fp_columns", 8)
+        if t.bdd_bp_staged and not values.get("bdd_bp_staged", 1):
+            values.setdefault("bdd_bp_zrun", min(t.bdd_bp_zrun, 8))
+        for k, v in values.items():
             if k not in t.as_dict():
                 raise KeyError(f"unknown tuning key {k!r}")
             setattr(t, k, int(v))

@@ -126,3 +126,39 @@ def test_invalid_shape_rejected(cuda, key, value):
     with pytest.raises(_native.NativeError):
         o.tuning = {key: value}
     assert o.tuning == before
+
+
+def test_unstaged_calls_run_the_unstaged_width(cuda):
+    """Where the default width is the staged kernels' 16, a call whose buffer is
+    off a 16-byte boundary, and a handle whose staging was switched off, run the
+    8-wide unstaged kernels (bit for bit), as they did before that default."""
+    import torch
+    from configs import apply
+    from omega_b200.projector import proj
+    nproj = 64 + 6 * torch.cuda.get_device_properties(cuda).multi_processor_count // 2
+    o = apply(proj.projectorClass(), dict(
+        CT=True, nRowsD=64, nColsD=64, nProjections=nproj, dPitchX=3.0, dPitchY=3.0, sourceToCRot=500.,
+        sourceToDetector=1000., Nx=192, Ny=192, Nz=64, FOVa_x=64., FOVa_y=64., axial_fov=64., projector_type=5,
+        subsets=1, subsetType=8, Niter=1, verbose=0,
+        angles=np.linspace(0, 2 * np.pi, nproj, endpoint=False).astype(np.float32),
+        SinM=np.zeros((64, 64, nproj), dtype=np.float32)))
+    o.addProjector()
+    o.initProj()
+    default = o.tuning
+    assert default["bdd_fp_columns"] == 16 and default["bdd_bp_zrun"] == 16
+    gen = torch.Generator(device=cuda).manual_seed(4)
+    rand = lambda n: torch.rand(n + 1, generator=gen, device=cuda)  # noqa: E731
+    xs, ys = rand(int(o.N[0])), rand(o.measurementCount(0))
+    x, y = xs[1:], ys[1:]   # 4 bytes off
+
+    def both():
+        return o.forwardProject(x, 0).clone(), o.backwardProject(y, 0).clone()
+    off = both()
+    o.tuning = {"bdd_fp_staged": 0, "bdd_bp_staged": 0}
+    assert o.tuning["bdd_fp_columns"] == 8 and o.tuning["bdd_bp_zrun"] == 8
+    alone = both()
+    o.tuning = {"bdd_fp_columns": 16, "bdd_bp_zrun": 16}
+    wide = both()
+    for a, b, c in zip(off, alone, wide):
+        assert torch.equal(a, b)
+        assert not torch.equal(b, c)   # (the widths add in another order)
