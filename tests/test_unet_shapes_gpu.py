@@ -1,7 +1,8 @@
 """The network's convolution, weight gradient and resampling kernels at the
 volumes where their tiles go wrong first: one voxel per axis, lines just below,
-at and above a tile's 128, partial tiles in every axis, against the FP64
-oracle / torch.  Bars: BF16 outputs 4e-3 relative L2 (half a unit in the last
+at and above a tile's 128, partial tiles, against the FP64 oracle / torch.
+(Volumes this small take one block of one line and one plane per thread block;
+test_unet_blocks_gpu.py has the larger ones.)  Bars: BF16 outputs 4e-3 relative L2 (half a unit in the last
 place is 2^-9), FP32 weight gradients 1e-5."""
 import ctypes
 
