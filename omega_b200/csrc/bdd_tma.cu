@@ -1,15 +1,16 @@
 // Type-5 (branchless distance-driven) forward projection with the image
 // patches staged by the tensor memory accelerator.
 //
-// Same per-ray arithmetic as k_bdd_fp<8> (bdd.cu): thread = (detector row,
-// group of 8 columns, projection), slices along the dominant source axis, one
-// row integral per voxel row the 8 column footprints cross.  What changes is
-// where the voxels come from.  A CTA covers 32 detector rows x kRB groups of 8
-// columns of one projection; on slice j its rays' footprints lie inside a
-// small box of the slice (lateral x z), found from the CTA's four corner rays
-// (the footprint edges are monotonic along the panel).  One thread per slice
-// loads that box with cp.async.bulk.tensor into a kStages-deep ring of
-// shared-memory buffers, kStages - 1 slices ahead of the compute, completing
+// Same per-ray arithmetic as k_bdd_fp<C> (bdd.cu): thread = (detector row,
+// group of C = 8 or 16 columns, projection), slices along the dominant source
+// axis, one row integral per voxel row the C column footprints cross.  What
+// changes is where the voxels come from.  A CTA covers 32 detector rows x 4
+// groups of C columns of one projection; on slice j its rays' footprints lie
+// inside a small box of the slice (lateral x z: 40 x 36 voxels for C = 8, 40 x
+// 60 for 16), found from the CTA's four corner rays (the footprint edges are
+// monotonic along the panel).  One thread per slice loads that box with
+// cp.async.bulk.tensor into a ring of 4 (C = 8) or 3 shared-memory buffers, one
+// slice less than that ahead of the compute, completing
 // on an mbarrier; the row integrals then read shared memory.  A ray whose
 // footprint leaves the box on some slice (geometries the box was not sized
 // for) reads that slice from global memory instead, with the same arithmetic,

@@ -108,7 +108,7 @@ struct Tof {
     const int *order;     // and which bin each one is
     float k2, kv, kq;     // exponents per mm^2 (base 2) and series scale of the window's weights
     int series;           // the weights' cosh series holds for every element
-    int window;           // bins a thread keeps (one of kTofWindows)
+    int window;           // bins a thread keeps (one of OMB_TOF_WINDOWS)
 };
 
 // Per-projection constants of the distance-driven backprojection: a
@@ -202,7 +202,7 @@ struct Tuning {
     int bdd_bp_rows = 8;            // type-5 backward: warps per block (4, 8)
     int siddon_layout = 1;          // frame batches: 0 = frame-major reads/atomics, 1 = voxel-interleaved
     int siddon_fp_steps = 4;        // non-TOF forward walks: crossings gathered per batched step (1, 2, 4)
-    int bdd_fp_staged = 1;          // type-5 forward: image boxes staged by TMA (with 8 columns per thread)
+    int bdd_fp_staged = 1;          // type-5 forward: image boxes staged by TMA (with 8 or 16 columns per thread)
     int bdd_bp_staged = 1;          // type-5 backward: detector boxes staged by TMA (with 8 or 16 voxels per thread)
     int siddon_bp_matrix = 0;       // type-1 non-TOF backprojection through a resident transposed system matrix
 };

@@ -19,8 +19,7 @@ namespace omb {
 // the traversal cost is shared by up to FB images.  Non-TOF forward walks are
 // latency-bound gathers: capping them at 64 registers (4 blocks, 32 warps per
 // SM) beats the spills it costs (measured: 30.6 -> 23.6 ms single-frame, 6.0
-// -> 3.9 ms for the interleaved 8-frame walk); the TOF variants keep their
-// registers (their weight arrays would spill hundreds of bytes).
+// -> 3.9 ms for the interleaved 8-frame walk).
 template <int FB, typename T, int K>
 __global__ void __launch_bounds__(kBlock, 4) k_siddon_fp(Grid g, RaySet rs, float gf, const T *__restrict__ img,
                                                          const T *__restrict__ imgT, int64_t img_stride,

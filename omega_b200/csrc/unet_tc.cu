@@ -678,10 +678,13 @@ __global__ void __launch_bounds__(256) k_conv3d_lines(const __grid_constant__ Li
 constexpr int kHalfSmem = 111 * 1024;
 
 // Block shape of a convolution: the least estimated time per output voxel over
-// the blocks that fit.  An instruction takes 32 clocks for its 4 KB of A plus
-// one per 4 columns; a staged 16-byte row costs the loaders about a third; two
-// CTAs on an SM (half the shared memory and tensor-memory columns each) hide
-// the epilogue, and a last wave that is partly empty counts in full.
+// the blocks that fit.  The estimate counts an instruction as 32 clocks for its
+// 4 KB of A plus one per 4 columns (timed alone it takes about 128 whatever its
+// columns, see k_conv3d_lines: the estimate leans to fewer columns, that is
+// planes, than that would; shapes planned with 128 have not been timed); a
+// staged 16-byte row costs the loaders about a third; two CTAs on an SM (half
+// the shared memory and tensor-memory columns each) hide the epilogue, and a
+// last wave that is partly empty counts in full.
 static ConvPlan conv_plan(int cin, int co, int groups, int X, int Y, int Z, int B) {
     ConvPlan best{};
     double best_cost = 1e300;
