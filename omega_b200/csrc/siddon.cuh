@@ -459,6 +459,10 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
         skip = pre_loop_2d(bx, bz, diff.x, diff.z, mx, mz, dxg, dzg, g.nx, g.nz, ti, tk, ax, az, np, s.x, s.z, d.x,
                            d.z, tcd);
         if (d.y > my || d.y < by) skip = true;
+        // End points equal in x and apart in y by less than 1e-6: the ray runs
+        // along z.  No sinogram bin has such a pair of crystals, so the TOF walk,
+        // whose elements must not be longer than a voxel's diagonal, leaves it out.
+        if (NB == 0 && isnan(ax.next())) skip = true;
     } else if (fabs(diff.x) < 1e-6) {
         ti = perpendicular_start(bx, d.x, dxg, g.nx);
         skip = pre_loop_2d(by, bz, diff.y, diff.z, my, mz, dyg, dzg, g.ny, g.nz, tj, tk, ay, az, np, s.y, s.z, d.y,
@@ -478,6 +482,19 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
     if constexpr (NB == 0) vis.begin(ddsign);
     float tc = (float)tcd;
     float tx = ax.next(), ty = ay.next(), tz = az.next();
+    int64_t ind = (int64_t)tj * sty + (int64_t)ti * stx + (int64_t)tk * nxy;
+    if constexpr (NB != 0) {
+        // A ray along z (list-mode events; see above) has no crossing in x, only
+        // 0 times infinity.  As in the reference's kernels its first voxel takes
+        // the rest of the ray; its steps would not end at `te` below.
+        if (isnan(tx + ty + tz)) {
+            const float ele = tc >= 0.f && tc <= 1.f ? (1.f - tc) * L : 0.f;
+            float tsum = 1.f;
+            if constexpr (NB > 1) tsum = tof_weights<NB>(tof, ddsign, ele, D, w);
+            vis(ind, ele, w, tsum);
+            return true;
+        }
+    }
     // The walk: every step takes the nearest of the three next crossings
     // without branching (the three outcomes diverge inside a warp otherwise;
     // issue slots bound the walks of one image: one 196,608-ray subset of 128 x
@@ -489,7 +506,6 @@ __device__ __forceinline__ bool siddon_walk(const Grid &g, const Ray &ray, bool 
     const float te = fminf(fminf(ax.leave(ti, g.nx), ay.leave(tj, g.ny)), az.leave(tk, g.nz));
     // both end points outside the grid (every scanner): no clamp to [0, 1]
     const bool through = tc >= 0.f && te <= 1.f;
-    int64_t ind = (int64_t)tj * sty + (int64_t)ti * stx + (int64_t)tk * nxy;
     const int dxi = ax.u * stx, dyi = ay.u * sty;
     const int64_t dzi = az.u * nxy;
     auto step = [&](float &ele) {
